@@ -34,6 +34,12 @@ struct NearPairV {
   long long dst[4];
 };
 
+// p2 x p2 block at scalar offset src of the dense-block pool (blocks of B rows,
+// column-major) whose transpose is the block at dst
+struct NearMirror {
+  long long src, dst;
+};
+
 // a Gauss point of the Maxwell quadrature tables: surface point, the two
 // tangents of the patch parametrisation and the weight h * w (no surface
 // measure: the vector basis carries the Jacobian)
@@ -58,6 +64,8 @@ cudaError_t launch_near_regular(int P, bool cplx, const NearPair* pairs, int npa
 cudaError_t launch_near_duffy(int G, int P, bool cplx, int cs, const PatchTable& pt, const ElementTable& et,
                               const NearPair* pairs, int npairs, const double* gx, const double* gw, int n1,
                               double kre, double kim, void* out, int B, cudaStream_t s);
+// transposed copies of finished element-pair blocks
+cudaError_t launch_near_mirror(bool cplx, const NearMirror* list, long n, int p2, int B, void* out, cudaStream_t s);
 
 // Maxwell single layer (Maxwell/SingleLayerOperator.hpp:44-88): the four
 // component blocks of every element pair, idiv = -1 / (kappa^2 h^2)
