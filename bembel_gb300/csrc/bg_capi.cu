@@ -918,6 +918,19 @@ std::vector<double> basis3_table(int P, const Rule1D& gr) {
 
 // Dense leaves of the Maxwell operator: every element pair fills its four
 // component blocks at once (H2Matrix.hpp:195-205 scatters them per component).
+// whether the swapped pair (class b) uses the same rule as the pair (class a)
+static bool same_rule_swapped(const PairClass& a, const PairClass& b) {
+  return a.cs == b.cs && a.deg == b.deg && (a.cs < 3 || (a.rot1 == b.rot2 && a.rot2 == b.rot1));
+}
+
+// first of block row r's blocks with column c among the rows' blocks of
+// component pair 0 (scalar operators: of all); -1 if none
+static long find_block(const BsrSegment& D, int r, int c) {
+  for (int k = D.row_ptr[r]; k < D.row_ptr[r + 1]; ++k)
+    if (D.col[k] == c && D.comp[k] == 0) return k;
+  return -1;
+}
+
 static bg_status assemble_near_mw(bg_operator* op) {
   cudaStream_t s = op->ctx->stream;
   const BsrSegment& D = op->dense;
@@ -936,6 +949,7 @@ static bg_status assemble_near_mw(bg_operator* op) {
   }
   std::map<int, std::vector<NearPairV>> regular;
   std::map<std::pair<int, int>, std::vector<NearPairV>> singular;
+  std::vector<NearMirror> mirrored;  // as near_work: block (cc, rc) of the swapped pair is the transpose
   long npairs = 0;
   for (int r = 0; r < ncl; ++r)
     for (int k = D.row_ptr[r]; k < D.row_ptr[r + 1]; ++k) {
@@ -944,6 +958,9 @@ static bg_status assemble_near_mw(bg_operator* op) {
       if (kk[0] < 0 || kk[1] < 0 || kk[2] < 0 || kk[3] < 0)
         return set_error(op->ctx, BG_DEVICE_ERROR, "incomplete component blocks of a dense leaf");
       const int c1 = r, c2 = D.col[k];
+      const long kt = find_block(D, c2, c1);
+      const std::array<long, 4> kkt = kt >= 0 ? where[D.leaf[kt]] : std::array<long, 4>{-1, -1, -1, -1};
+      const bool twin = kkt[0] >= 0 && kkt[1] >= 0 && kkt[2] >= 0 && kkt[3] >= 0;
       for (int b = 0; b < ecl; ++b)
         for (int a = 0; a < ecl; ++a) {
           const int e1 = c1 * ecl + a, e2 = c2 * ecl + b;
@@ -954,6 +971,14 @@ static bg_status assemble_near_mw(bg_operator* op) {
           np.rot = (pc.rot1 & 15) | ((pc.rot2 & 15) << 4);
           np.pad = 0;
           for (int c = 0; c < 4; ++c) np.dst[c] = (long long)kk[c] * bstride + (long long)(b * p2) * B + a * p2;
+          if (twin && e1 > e2 && same_rule_swapped(pc, classify_pair(op->mesh, e2, e1, op->P))) {
+            for (int c = 0; c < 4; ++c) {
+              const int ct = ((c & 1) << 1) | (c >> 1);  // (cc, rc)
+              mirrored.push_back({(long long)kkt[ct] * bstride + (long long)(a * p2) * B + b * p2, np.dst[c]});
+            }
+            ++npairs;
+            continue;
+          }
           if (pc.cs == 0) regular[pc.deg].push_back(np);
           else singular[{pc.cs, pc.deg}].push_back(np);
           ++npairs;
@@ -975,19 +1000,6 @@ static bg_status assemble_near_mw(bg_operator* op) {
   bg_status st = BG_OK;
   for (auto& kv : regular) {
     const int deg = kv.first, n1 = deg + 1, Q = n1 * n1;
-// whether the swapped pair (class b) uses the same rule as the pair (class a)
-static bool same_rule_swapped(const PairClass& a, const PairClass& b) {
-  return a.cs == b.cs && a.deg == b.deg && (a.cs < 3 || (a.rot1 == b.rot2 && a.rot2 == b.rot1));
-}
-
-// first of block row r's blocks with column c among the rows' blocks of
-// component pair 0 (scalar operators: of all); -1 if none
-static long find_block(const BsrSegment& D, int r, int c) {
-  for (int k = D.row_ptr[r]; k < D.row_ptr[r + 1]; ++k)
-    if (D.col[k] == c && D.comp[k] == 0) return k;
-  return -1;
-}
-
     const Rule1D& gr = gauss_rule(n1);
     const std::vector<double> basis3 = basis3_table(P, gr);
     DevBuf *dgx = new DevBuf(), *dgw = new DevBuf(), *dtab = new DevBuf(), *dbas = new DevBuf(), *dpairs = new DevBuf();
@@ -1006,7 +1018,6 @@ static long find_block(const BsrSegment& D, int r, int c) {
       cleanup();
       return st;
     }
-  std::vector<NearMirror> mirrored;  // as near_work: block (cc, rc) of the swapped pair is the transpose
   }
   for (auto& kv : singular) {
     const int cs = kv.first.first, deg = kv.first.second, n1 = deg + 1;
@@ -1015,9 +1026,6 @@ static long find_block(const BsrSegment& D, int r, int c) {
     keep.insert(keep.end(), {dgx, dgw, dpairs});
     cudaError_t e = dgx->upload(gr.x, s);
     if (e == cudaSuccess) e = dgw->upload(gr.w, s);
-      const long kt = find_block(D, c2, c1);
-      const std::array<long, 4> kkt = kt >= 0 ? where[D.leaf[kt]] : std::array<long, 4>{-1, -1, -1, -1};
-      const bool twin = kkt[0] >= 0 && kkt[1] >= 0 && kkt[2] >= 0 && kkt[3] >= 0;
     if (e == cudaSuccess) e = dpairs->upload(kv.second, s);
     if (e == cudaSuccess)
       e = launch_near_duffy_mw(op->G, P, cs, pt, et, dpairs->as<NearPairV>(), (int)kv.second.size(),
@@ -1027,20 +1035,10 @@ static long find_block(const BsrSegment& D, int r, int c) {
       return st;
     }
   }
-  // the swapped pairs, once every block they are copied from is complete
   DevBuf dmirror;
-  cudaError_t e = dmirror.upload(w.mirrored, s);
-  for (int q = 0; q < nk && e == cudaSuccess; ++q)
-    e = launch_near_mirror(op->cplx, dmirror.as<NearMirror>(), (long)w.mirrored.size(), p2, B, out[q], s);
+  cudaError_t e = dmirror.upload(mirrored, s);
+  if (e == cudaSuccess) e = launch_near_mirror(true, dmirror.as<NearMirror>(), (long)mirrored.size(), p2, B, out, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-          if (twin && e1 > e2 && same_rule_swapped(pc, classify_pair(op->mesh, e2, e1, op->P))) {
-            for (int c = 0; c < 4; ++c) {
-              const int ct = ((c & 1) << 1) | (c >> 1);  // (cc, rc)
-              mirrored.push_back({(long long)kkt[ct] * bstride + (long long)(a * p2) * B + b * p2, np.dst[c]});
-            }
-            ++npairs;
-            continue;
-          }
   cleanup();
   return cuda_status(op->ctx, e, "near-field assembly");
 }
@@ -1048,9 +1046,17 @@ static long find_block(const BsrSegment& D, int r, int c) {
 // Element pairs of the dense leaves of a scalar operator, classified on the
 // host (FP64, as the reference): regular pairs by quadrature degree, singular
 // pairs by (case, degree); dst is the entry offset of the pair's block.
+//
+// The rules are symmetric under exchange of the two elements (the Gauss rules
+// and the Duffy maps of a pair and of the swapped pair are the same points),
+// and so is the kernel, so the block of (e2, e1) is the transpose of that of
+// (e1, e2) to rounding (2e-15 in the oracle). With `mirror`, pairs e1 > e2
+// whose swapped pair is classified alike (case, degree and orientations) are
+// left out of the rules and copied instead (mirrored: transposed copy).
 struct NearWork {
   std::map<int, std::vector<NearPair>> regular;
   std::map<std::pair<int, int>, std::vector<NearPair>> singular;
+  std::vector<NearMirror> mirrored;
   long npairs = 0;
 };
 
@@ -1062,6 +1068,7 @@ static NearWork near_work(const bg_operator* op, bool mirror) {
   for (int r = 0; r < D.nrows; ++r)
     for (int k = D.row_ptr[r]; k < D.row_ptr[r + 1]; ++k) {
       const int c1 = r, c2 = D.col[k];
+      const long kt = mirror ? find_block(D, c2, c1) : -1;
       for (int b = 0; b < ecl; ++b)
         for (int a = 0; a < ecl; ++a) {
           const int e1 = c1 * ecl + a, e2 = c2 * ecl + b;
@@ -1072,6 +1079,11 @@ static NearWork near_work(const bg_operator* op, bool mirror) {
           np.rot = (pc.rot1 & 15) | ((pc.rot2 & 15) << 4);
           np.pad = 0;
           np.dst = (long long)k * bstride + (long long)(b * p2) * B + a * p2;
+          ++w.npairs;
+          if (kt >= 0 && e1 > e2 && same_rule_swapped(pc, classify_pair(op->mesh, e2, e1, op->P))) {
+            w.mirrored.push_back({(long long)kt * bstride + (long long)(a * p2) * B + b * p2, np.dst});
+            continue;
+          }
           if (pc.cs == 0) w.regular[pc.deg].push_back(np);
           else w.singular[{pc.cs, pc.deg}].push_back(np);
         }
@@ -1108,17 +1120,9 @@ static bg_status near_quadrature(bg_operator* op, const NearWork& w, int nk, con
         for (int ix = 0; ix <= op->P; ++ix) basis[(size_t)q * p2 + iy * (op->P + 1) + ix] = bs[ix] * bt[iy];
     }
     DevBuf *dgx = new DevBuf(), *dgw = new DevBuf(), *dtab = new DevBuf(), *dbas = new DevBuf(), *dpairs = new DevBuf();
-//
-// The rules are symmetric under exchange of the two elements (the Gauss rules
-// and the Duffy maps of a pair and of the swapped pair are the same points),
-// and so is the kernel, so the block of (e2, e1) is the transpose of that of
-// (e1, e2) to rounding (2e-15 in the oracle). With `mirror`, pairs e1 > e2
-// whose swapped pair is classified alike (case, degree and orientations) are
-// left out of the rules and copied instead (mirrored: transposed copy).
     keep.insert(keep.end(), {dgx, dgw, dtab, dbas, dpairs});
     cudaError_t e = dgx->upload(gr.x, s);
     if (e == cudaSuccess) e = dgw->upload(gr.w, s);
-  std::vector<NearMirror> mirrored;
     if (e == cudaSuccess) e = dbas->upload(basis, s);
     if (e == cudaSuccess) e = dpairs->upload(kv.second, s);
     if (e == cudaSuccess) e = dtab->alloc((size_t)op->ne * Q * sizeof(d4));
@@ -1129,7 +1133,6 @@ static bg_status near_quadrature(bg_operator* op, const NearWork& w, int nk, con
     if ((st = cuda_status(op->ctx, e, "near-field regular pairs")) != BG_OK) {
       cleanup();
       return st;
-      const long kt = mirror ? find_block(D, c2, c1) : -1;
     }
   }
   const bool multi = op->cplx && nk > 1 && (op->P == 1 || op->P == 2);
@@ -1140,11 +1143,6 @@ static bg_status near_quadrature(bg_operator* op, const NearWork& w, int nk, con
     keep.insert(keep.end(), {dgx, dgw, dpairs});
     cudaError_t e = dgx->upload(gr.x, s);
     if (e == cudaSuccess) e = dgw->upload(gr.w, s);
-          ++w.npairs;
-          if (kt >= 0 && e1 > e2 && same_rule_swapped(pc, classify_pair(op->mesh, e2, e1, op->P))) {
-            w.mirrored.push_back({(long long)kt * bstride + (long long)(a * p2) * B + b * p2, np.dst});
-            continue;
-          }
     if (e == cudaSuccess) e = dpairs->upload(kv.second, s);
     // the common-edge and common-vertex rules have factorised one-wavenumber
     // kernels (P <= 2, n1 <= 16), faster than sharing per-sample work over
@@ -1166,9 +1164,11 @@ static bg_status near_quadrature(bg_operator* op, const NearWork& w, int nk, con
       return st;
     }
   }
+  // the swapped pairs, once every block they are copied from is complete
   DevBuf dmirror;
-  cudaError_t e = dmirror.upload(mirrored, s);
-  if (e == cudaSuccess) e = launch_near_mirror(true, dmirror.as<NearMirror>(), (long)mirrored.size(), p2, B, out, s);
+  cudaError_t e = dmirror.upload(w.mirrored, s);
+  for (int q = 0; q < nk && e == cudaSuccess; ++q)
+    e = launch_near_mirror(op->cplx, dmirror.as<NearMirror>(), (long)w.mirrored.size(), p2, B, out[q], s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   cleanup();
   return cuda_status(op->ctx, e, "near-field assembly");
@@ -1191,7 +1191,7 @@ static bg_status assemble_near(bg_operator* op) {
       return BG_OK;
     }
   BG_CHECK(cudaMemsetAsync(op->d_dense64.p, 0, bytes, s), "near-field storage");
-  const NearWork w = near_work(op, false);
+  const NearWork w = near_work(op, true);
   op->near_pairs = w.npairs;
   void* out = op->d_dense64.p;
   return near_quadrature(op, w, 1, &op->kre, &op->kim, &out);
@@ -1202,7 +1202,7 @@ extern "C" bg_status bg_operator_quadrature_counts(const bg_operator* op, long* 
   for (int i = 0; i < 8; ++i) counts8[i] = 0;
   if (op->maxwell() || op->vd != 1)
     return set_error(op->ctx, BG_UNSUPPORTED, "quadrature counts: scalar operators only");
-  const NearWork w = near_work(op, true);
+  const NearWork w = near_work(op, false);
   for (const auto& kv : w.regular) {
     const long q = (long)(kv.first + 1) * (kv.first + 1);
     counts8[0] += (long)kv.second.size();
