@@ -484,6 +484,20 @@ static bg_status upload_tables(bg_operator* op) {
       }
     }
   }
+  auto longest = [](const BsrSegment& f) {
+    int m = 0;
+    for (int r = 0; r < f.nrows; ++r) m = std::max(m, f.row_ptr[r + 1] - f.row_ptr[r]);
+    return m;
+  };
+  op->near_row_max = longest(op->dense);
+  op->far_row_max = 0;
+  for (const auto& f : op->far) op->far_row_max = std::max(op->far_row_max, longest(f));
+  // FP64-accurate products on the tensor cores: leaf blocks and clusters of at
+  // most 128 rows, rows within the fixed point of the sums
+  op->near_oz = !op->dense.col.empty() && (long)op->dense.nrows * op->dense.B == (long)op->S &&
+                bsr_oz_supported(op->dense.B, op->cplx, false, op->near_row_max);
+  op->far_oz = op->far_row_max > 0 && op->leaf_level < kOzMaxSegs &&
+               bsr_oz_supported(op->far[0].B, op->cplx, true, op->far_row_max);
   {
     // every row of every far-field level, rows with more blocks first so the
     // longest CTAs start in the first wave
@@ -637,13 +651,22 @@ extern "C" bg_status bg_watchdog_selftest(bg_context* ctx, long long limit_cycle
 }
 #undef WD_CHECK
 
+// Passes of 32 columns (complex: 16) of the FP64-accurate tensor-core product
+// that run in one launch and hold their digit panels side by side: two where
+// one pass has fewer than four block rows per SM, whose persistent CTAs would
+// run out of rows unevenly.
+static int oz_passes(const bg_operator* op, int nrows, int ncols) {
+  const int per = op->cplx ? 16 : 32;
+  return ncols > per && nrows < 4 * 152 ? 2 : 1;
+}
+
 extern "C" bg_status bg_operator_memory(const bg_operator* op, size_t* allocated, size_t* estimate) {
   if (!op || !allocated || !estimate) return BG_INVALID_ARG;
   size_t a = 0;
   for (const DevBuf* b : {&op->d_patch_meta, &op->d_patch_cp, &op->d_el_patch, &op->d_el_llc, &op->d_T_ptr,
                           &op->d_T_idx, &op->d_T_val, &op->d_Tt_ptr, &op->d_Tt_idx, &op->d_Tt_val, &op->d_cheb,
-                          &op->d_dense64, &op->d_dense32, &op->d_dense_df, &op->d_oz_tiles, &op->d_oz_rexp,
-                          &op->w_oz_panels, &op->w_oz_fmax, &op->d_tr64, &op->d_tr32,
+                          &op->d_dense64, &op->d_dense32, &op->d_dense_df, &op->d_dense_dig, &op->w_oz_near,
+                          &op->w_oz_far, &op->w_oz_fmax, &op->d_tr64, &op->d_tr32,
                           &op->d_far_work, &op->d_err, &op->w_xdof, &op->w_xss, &op->w_yss, &op->w_ydof,
                           &op->w_xss32, &op->w_yss32, &op->w_xss_df,
                           &op->dense.d_row_ptr, &op->dense.d_col})
@@ -660,7 +683,7 @@ extern "C" bg_status bg_operator_memory(const bg_operator* op, size_t* allocated
   for (const auto& c : op->near_cache) a += c.blocks->bytes;
   for (const auto& k : op->kslots) {  // batched wavenumbers (the active slot's fields are counted above)
     if (&k == &op->kslots[0] + op->kslot_active) continue;
-    a += k.dense64.bytes + k.dense32.bytes;
+    a += k.dense64.bytes + k.dense32.bytes + k.dense_dig.bytes;
     for (const auto* v : {&k.far64, &k.far_df, &k.atiles, &k.ainv})
       for (const DevBuf* b : *v) a += b->bytes;
   }
@@ -673,16 +696,18 @@ extern "C" bg_status bg_operator_memory(const bg_operator* op, size_t* allocated
   size_t e = (size_t)op->dense.col.size() * op->block_stride(op->dense.B) * sb +
              (size_t)op->dense.col.size() * op->block_stride32(op->dense.B) * sb / 2;
   if (!op->cplx) e += (size_t)op->dense.col.size() * op->block_stride(op->dense.B) * sizeof(float2);  // double-float
-  if (!op->cplx && oz_supported(op->dense.B))  // tensor-core digit tiles, row exponents, x digit panels
-    e += oz_tile_bytes(op->dense.B, (long)op->dense.col.size()) + (size_t)op->dense.nrows * op->dense.B * sizeof(int) +
-         oz_panel_bytes(op->dense.B, op->S / op->dense.B) + 32 * sizeof(int);
+  if (op->near_oz)  // digit bytes, row exponents, x digit panels
+    e += (op->cplx ? 0 : op->digit_bytes((long)op->dense.col.size(), op->dense.B)) +
+         (size_t)op->dense.nrows * op->dense.B * sizeof(int) + (size_t)op->dense.nrows * bsr_oz_panel_bytes(op->dense.B, op->cplx) * oz_passes(op, op->dense.nrows, 32);
   for (int l = 0; l <= op->leaf_level && l < (int)op->far.size(); ++l) {
     const size_t nb = op->far[l].col.size();
     const size_t ncl = (size_t)op->nclusters(l);
     e += ncl * np2 * (sizeof(d4) + sizeof(float4) + (op->maxwell() ? 6 * (sizeof(double) + sizeof(float)) : 0));
     if (!op->store_far) continue;
     if (op->keep_far64) e += nb * op->block_stride(op->far[l].B) * sb;  // FP64 couplings
-    e += nb * op->block_stride(op->far[l].B) * 8 * (op->cplx ? 2 : 1);  // double-float pairs
+    e += nb * op->block_stride(op->far[l].B) * 8 * (op->cplx ? 2 : 1);  // digit bytes or double-float pairs
+    if (nb > 0 && op->far_oz)  // row exponents, x digit panels
+      e += (size_t)op->far[l].nrows * op->far[l].B * sizeof(int) + ncl * bsr_oz_panel_bytes(op->far[l].B, op->cplx) * oz_passes(op, op->n_far_work, 32);
     e += nb * (op->cplx ? far_h16c_atile_bytes(np2) : far_h16_atile_bytes(np2)) + nb * sizeof(float);
   }
   // work vectors and solver workspaces for 32 right-hand sides: superspace and
@@ -800,6 +825,58 @@ extern "C" bg_status bg_operator_leaf_block(const bg_operator* op, long leaf, in
 
 // ---------------------------------------------------------------------------
 // Assembly (H2Matrix::init_H2Matrix, H2Matrix.hpp:93-250)
+// A far-field level with couplings df, and the near field with blocks dense64
+// and digits dig, as segments of the FP64-accurate tensor-core product
+static OzSeg oz_far_seg(const bg_operator* op, int l, const DevBuf* df, const void* x, void* y, unsigned char* panels) {
+  const BsrSegment& f = op->far[l];
+  OzSeg g{};
+  g.row_ptr = f.d_row_ptr.as<int>();
+  g.col = f.d_col.as<int>();
+  g.tstride = bsr_oz_tile_stride(f.B);  // digit bytes and pairs alike
+  g.im_off = (long)f.col.size() * g.tstride;
+  if (!f.col.empty()) {
+    g.tiles = df->as<unsigned char>();
+    g.rexp = reinterpret_cast<const int*>(g.tiles + op->digit_bytes((long)f.col.size(), f.B));
+    g.ncl = op->nclusters(l);
+  }
+  g.x = static_cast<const double*>(x);
+  g.y = static_cast<double*>(y);
+  g.panels = panels;
+  return g;
+}
+OzSeg oz_far_seg(const bg_operator* op, int l, const void* x, void* y) {
+  return oz_far_seg(op, l, op->d_far_df[l], x, y, nullptr);
+}
+static OzSeg oz_near_seg(const bg_operator* op, const DevBuf& dense64, const DevBuf& dig) {
+  const BsrSegment& f = op->dense;
+  OzSeg g{};
+  g.row_ptr = f.d_row_ptr.as<int>();
+  g.col = f.d_col.as<int>();
+  g.tiles = op->cplx ? dense64.as<unsigned char>() : dig.as<unsigned char>();
+  g.tstride = op->cplx ? op->block_stride(f.B) * 16 : bsr_oz_tile_stride(f.B);
+  g.rexp = reinterpret_cast<const int*>(dig.as<unsigned char>() +
+                                        (op->cplx ? 0 : op->digit_bytes((long)f.col.size(), f.B)));
+  g.ncl = f.nrows;
+  g.x = op->w_xss.as<double>();
+  g.y = op->w_yss.as<double>();
+  g.panels = op->w_oz_near.as<unsigned char>();
+  return g;
+}
+// row exponents of segment f (FP64 blocks) and, for real operators, digit
+// bytes into dig, the exponents behind ahead bytes
+static cudaError_t build_digits(bg_operator* op, const BsrSegment& f, const void* blocks, DevBuf* dig, size_t ahead) {
+  cudaError_t e = dig->alloc(ahead + (size_t)f.nrows * f.B * sizeof(int));
+  if (e != cudaSuccess) return e;
+  unsigned char* t = dig->as<unsigned char>();
+  int* rexp = reinterpret_cast<int*>(t + ahead);
+  cudaStream_t s = op->ctx->stream;
+  const long bs = op->block_stride(f.B);
+  e = launch_bsr_oz_rows(op->cplx, f.d_row_ptr.as<int>(), blocks, bs, f.nrows, f.B, rexp, s);
+  if (e == cudaSuccess && !op->cplx)
+    e = launch_bsr_oz_tiles(f.d_row_ptr.as<int>(), static_cast<const double*>(blocks), bs, f.nrows, f.B, rexp, t, s);
+  return e;
+}
+
 static bg_status assemble_far(bg_operator* op) {
   cudaStream_t s = op->ctx->stream;
   PatchTable pt{op->d_patch_meta.as<int>(), op->d_patch_cp.as<double>()};
@@ -855,7 +932,9 @@ static bg_status assemble_far(bg_operator* op) {
     if (op->cplx) {
       // double-float pairs of Re and Im for the complex FP64 product
       const long sdf = ((long)f.B * f.B + 1) / 2 * 2;
-      BG_CHECK(op->d_far_df[l]->alloc(2 * f.col.size() * sdf * sizeof(float2)), "far field storage");
+      const size_t ahead = op->digit_bytes((long)f.col.size(), f.B);
+      if (op->far_oz) BG_CHECK(build_digits(op, f, op->d_far64[l]->p, op->d_far_df[l], ahead), "far-field exponents");
+      else BG_CHECK(op->d_far_df[l]->alloc(ahead), "far field storage");
       BG_CHECK(launch_split_df_cplx_blocks(op->d_far64[l]->p, op->block_stride(f.B), (long)f.B * f.B, (long)f.col.size(),
                                            sdf, op->d_far_df[l]->p, s),
                "far-field split");
@@ -870,9 +949,13 @@ static bg_status assemble_far(bg_operator* op) {
         ++tiled_levels;
       }
     } else {
-      // (hi, lo) FP32 pairs of the same blocks for the double-float FP64 product
-      BG_CHECK(op->d_far_df[l]->alloc(bytes), "far field storage");
-      BG_CHECK(launch_split_df(op->d_far64[l]->p, (long)f.col.size() * op->block_stride(f.B), op->d_far_df[l]->p, s),
+      // digits, or (hi, lo) FP32 pairs, of the same blocks for the FP64 product
+      if (op->far_digits())
+        BG_CHECK(build_digits(op, f, op->d_far64[l]->p, op->d_far_df[l], op->digit_bytes((long)f.col.size(), f.B)),
+                 "far-field digits");
+      else BG_CHECK(op->d_far_df[l]->alloc(bytes), "far field storage");
+      if (!op->far_digits())
+        BG_CHECK(launch_split_df(op->d_far64[l]->p, (long)f.col.size() * op->block_stride(f.B), op->d_far_df[l]->p, s),
                "far-field split");
       // scaled FP16 hi / lo tiles in the tensor-core operand layout
       const size_t tb = far_h16_atile_bytes(np2);
@@ -886,7 +969,7 @@ static bg_status assemble_far(bg_operator* op) {
       }
     }
     BG_CHECK(cudaStreamSynchronize(s), "far-field assembly");
-    // the products read the double-float pairs and the tiles, not the FP64 blocks
+    // the products read the digits (or pairs) and the tiles, not the FP64 blocks
     if (!op->keep_far64 && op->d_far_df[l]->p) op->d_far64[l]->release();
   }
   op->far_tiles = tiled_levels == far_levels && op->leaf_level < kMaxFarLevels;
@@ -918,19 +1001,6 @@ std::vector<double> basis3_table(int P, const Rule1D& gr) {
 
 // Dense leaves of the Maxwell operator: every element pair fills its four
 // component blocks at once (H2Matrix.hpp:195-205 scatters them per component).
-// whether the swapped pair (class b) uses the same rule as the pair (class a)
-static bool same_rule_swapped(const PairClass& a, const PairClass& b) {
-  return a.cs == b.cs && a.deg == b.deg && (a.cs < 3 || (a.rot1 == b.rot2 && a.rot2 == b.rot1));
-}
-
-// first of block row r's blocks with column c among the rows' blocks of
-// component pair 0 (scalar operators: of all); -1 if none
-static long find_block(const BsrSegment& D, int r, int c) {
-  for (int k = D.row_ptr[r]; k < D.row_ptr[r + 1]; ++k)
-    if (D.col[k] == c && D.comp[k] == 0) return k;
-  return -1;
-}
-
 static bg_status assemble_near_mw(bg_operator* op) {
   cudaStream_t s = op->ctx->stream;
   const BsrSegment& D = op->dense;
@@ -949,7 +1019,6 @@ static bg_status assemble_near_mw(bg_operator* op) {
   }
   std::map<int, std::vector<NearPairV>> regular;
   std::map<std::pair<int, int>, std::vector<NearPairV>> singular;
-  std::vector<NearMirror> mirrored;  // as near_work: block (cc, rc) of the swapped pair is the transpose
   long npairs = 0;
   for (int r = 0; r < ncl; ++r)
     for (int k = D.row_ptr[r]; k < D.row_ptr[r + 1]; ++k) {
@@ -958,9 +1027,6 @@ static bg_status assemble_near_mw(bg_operator* op) {
       if (kk[0] < 0 || kk[1] < 0 || kk[2] < 0 || kk[3] < 0)
         return set_error(op->ctx, BG_DEVICE_ERROR, "incomplete component blocks of a dense leaf");
       const int c1 = r, c2 = D.col[k];
-      const long kt = find_block(D, c2, c1);
-      const std::array<long, 4> kkt = kt >= 0 ? where[D.leaf[kt]] : std::array<long, 4>{-1, -1, -1, -1};
-      const bool twin = kkt[0] >= 0 && kkt[1] >= 0 && kkt[2] >= 0 && kkt[3] >= 0;
       for (int b = 0; b < ecl; ++b)
         for (int a = 0; a < ecl; ++a) {
           const int e1 = c1 * ecl + a, e2 = c2 * ecl + b;
@@ -971,14 +1037,6 @@ static bg_status assemble_near_mw(bg_operator* op) {
           np.rot = (pc.rot1 & 15) | ((pc.rot2 & 15) << 4);
           np.pad = 0;
           for (int c = 0; c < 4; ++c) np.dst[c] = (long long)kk[c] * bstride + (long long)(b * p2) * B + a * p2;
-          if (twin && e1 > e2 && same_rule_swapped(pc, classify_pair(op->mesh, e2, e1, op->P))) {
-            for (int c = 0; c < 4; ++c) {
-              const int ct = ((c & 1) << 1) | (c >> 1);  // (cc, rc)
-              mirrored.push_back({(long long)kkt[ct] * bstride + (long long)(a * p2) * B + b * p2, np.dst[c]});
-            }
-            ++npairs;
-            continue;
-          }
           if (pc.cs == 0) regular[pc.deg].push_back(np);
           else singular[{pc.cs, pc.deg}].push_back(np);
           ++npairs;
@@ -1035,10 +1093,7 @@ static bg_status assemble_near_mw(bg_operator* op) {
       return st;
     }
   }
-  DevBuf dmirror;
-  cudaError_t e = dmirror.upload(mirrored, s);
-  if (e == cudaSuccess) e = launch_near_mirror(true, dmirror.as<NearMirror>(), (long)mirrored.size(), p2, B, out, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaError_t e = cudaStreamSynchronize(s);
   cleanup();
   return cuda_status(op->ctx, e, "near-field assembly");
 }
@@ -1053,12 +1108,27 @@ static bg_status assemble_near_mw(bg_operator* op) {
 // (e1, e2) to rounding (2e-15 in the oracle). With `mirror`, pairs e1 > e2
 // whose swapped pair is classified alike (case, degree and orientations) are
 // left out of the rules and copied instead (mirrored: transposed copy).
+// Maxwell's pairs are all integrated: its solves with an FP32 inner operator
+// turn a change of 1e-16 in the blocks into one of the stopping residual's
+// size in x.
 struct NearWork {
   std::map<int, std::vector<NearPair>> regular;
   std::map<std::pair<int, int>, std::vector<NearPair>> singular;
   std::vector<NearMirror> mirrored;
   long npairs = 0;
 };
+
+// whether the swapped pair (class b) uses the same rule as the pair (class a)
+static bool same_rule_swapped(const PairClass& a, const PairClass& b) {
+  return a.cs == b.cs && a.deg == b.deg && (a.cs < 3 || (a.rot1 == b.rot2 && a.rot2 == b.rot1));
+}
+
+// block row r's block with column c, -1 if none
+static long find_block(const BsrSegment& D, int r, int c) {
+  for (int k = D.row_ptr[r]; k < D.row_ptr[r + 1]; ++k)
+    if (D.col[k] == c) return k;
+  return -1;
+}
 
 static NearWork near_work(const bg_operator* op, bool mirror) {
   NearWork w;
@@ -1353,6 +1423,7 @@ extern "C" bg_status bg_operator_assemble_wavenumbers(bg_operator* op) {
     slot.kim = k.second;
     std::swap(slot.dense64, op->d_dense64);
     std::swap(slot.dense32, op->d_dense32);
+    std::swap(slot.dense_dig, op->d_dense_dig);
     std::swap(slot.far64, op->d_far64);
     std::swap(slot.far_df, op->d_far_df);
     std::swap(slot.atiles, op->d_far_atiles);
@@ -1409,6 +1480,7 @@ static void fresh_far_fields(bg_operator* op) {
   op->far_tiles = false;
   op->d_dense64.release();
   op->d_dense32.release();
+  op->d_dense_dig.release();
 }
 
 extern "C" bg_status bg_operator_assemble(bg_operator* op) {
@@ -1449,21 +1521,12 @@ extern "C" bg_status bg_operator_assemble(bg_operator* op) {
       if (e == cudaSuccess) e = cudaStreamSynchronize(op->ctx->stream);
       if ((st = cuda_status(op->ctx, e, "double-float near field")) != BG_OK) return st;
     }
-    // integer digits of the real blocks for the tensor-core near field of
-    // BG_PREC_MIXED products (and their per-product scratch: x digit panels,
-    // zero where no digit is written, and column exponents)
-    if (!op->cplx && nb > 0 && oz_supported((int)B) && (long)op->dense.nrows * B == (long)op->S) {
-      const int nrows = op->dense.nrows;
-      e = op->d_oz_tiles.alloc(oz_tile_bytes((int)B, nb));
-      if (e == cudaSuccess) e = op->d_oz_rexp.alloc((size_t)nrows * B * sizeof(int));
-      if (e == cudaSuccess) e = op->w_oz_panels.alloc(oz_panel_bytes((int)B, op->S / B));
-      if (e == cudaSuccess) e = op->w_oz_fmax.alloc(32 * sizeof(int));
-      if (e == cudaSuccess) e = cudaMemsetAsync(op->w_oz_panels.p, 0, op->w_oz_panels.bytes, op->ctx->stream);
-      if (e == cudaSuccess)
-        e = launch_oz_build(op->dense.d_row_ptr.as<int>(), op->d_dense64.as<double>(), op->block_stride((int)B), nrows,
-                            (int)B, op->d_oz_rexp.as<int>(), op->d_oz_tiles.p, nb, op->ctx->stream);
+    // digits (complex: row exponents) of the blocks for the FP64-accurate tensor-core product
+    if (nb > 0 && op->near_oz) {
+      e = build_digits(op, op->dense, op->d_dense64.p, &op->d_dense_dig,
+                       op->cplx ? 0 : op->digit_bytes(nb, (int)B));
       if (e == cudaSuccess) e = cudaStreamSynchronize(op->ctx->stream);
-      if ((st = cuda_status(op->ctx, e, "tensor-core near field digits")) != BG_OK) return st;
+      if ((st = cuda_status(op->ctx, e, "near-field digits")) != BG_OK) return st;
     }
   }
   auto t2 = std::chrono::steady_clock::now();
@@ -1475,6 +1538,61 @@ extern "C" bg_status bg_operator_assemble(bg_operator* op) {
 }
 
 // ---------------------------------------------------------------------------
+// bytes of one pass of the far field's digit panels; off: the levels' offsets in it
+static size_t oz_far_panels(const bg_operator* op, size_t* off) {
+  size_t n = 0;
+  for (int l = 0; l <= op->leaf_level; ++l) {
+    if (off) off[l] = n;
+    if (!op->far[l].col.empty()) n += bsr_oz_panel_bytes(op->far[l].B, op->cplx) * op->nclusters(l);
+  }
+  return n;
+}
+// Whether a near-field product with nc columns goes through the digits. A
+// digit product costs about the same up to 32 columns (complex: 16) and three
+// small launches more; the FP64 pipe is quicker for a single vector, and for
+// two with small blocks (sphere M = 4, B = 36, one column: 43 against 68 us,
+// two: 69 against 68; M = 5, P = 1, B = 16: 31 and 48 against 124 us; torus
+// M = 3, complex, one column: 293 against 289 us, Maxwell sphere M = 3: 150
+// against 177 us, two: 515 and 262 against 289 and 178 us).
+static bool near_by_digits(const bg_operator* op, const DevBuf& dig, int nc, bool solver) {
+  if (!op->near_oz || !dig.p || (solver && op->maxwell())) return false;
+  return nc > 2 || (nc == 2 && (op->cplx || op->dense.B > 16));
+}
+// columns c0 .. c0 + nc - 1 (rows of ld scalars) of the near field
+static cudaError_t oz_near_product(const bg_operator* op, const DevBuf& dense64, const DevBuf& dig, int ld, int c0, int nc) {
+  OzArgs a{};
+  a.seg[0] = oz_near_seg(op, dense64, dig);
+  a.nseg = 1;
+  a.nwork = op->dense.nrows;
+  a.B = op->dense.B;
+  a.ldx = ld;
+  a.c0 = c0;
+  a.ncols = nc;
+  a.pass_panels = (size_t)op->dense.nrows * bsr_oz_panel_bytes(a.B, op->cplx);
+  a.fmax = op->w_oz_fmax.as<int>();
+  a.err = op->d_err.as<int>();
+  return launch_bsr_oz(op->cplx, false, a, op->near_row_max, op->oz_near_passes, op->ctx->stream);
+}
+// the far field of every level with couplings df, y[l] to z[l]
+static cudaError_t oz_far_product(const bg_operator* op, const std::vector<DevBuf*>& df, const std::vector<DevBuf*>& y,
+                                  const std::vector<DevBuf*>& z, int ld, int c0, int nc) {
+  OzArgs a{};
+  size_t off[kOzMaxSegs];
+  a.pass_panels = oz_far_panels(op, off);
+  a.nseg = op->leaf_level + 1;
+  for (int l = 0; l <= op->leaf_level; ++l)
+    a.seg[l] = oz_far_seg(op, l, df[l], y[l]->p, z[l]->p, op->w_oz_far.as<unsigned char>() + off[l]);
+  a.work = op->d_far_work.as<int2>();
+  a.nwork = op->n_far_work;
+  a.B = op->far[0].B;
+  a.ldx = ld;
+  a.c0 = c0;
+  a.ncols = nc;
+  a.fmax = op->w_oz_fmax.as<int>();
+  a.err = op->d_err.as<int>();
+  return launch_bsr_oz(op->cplx, op->cplx, a, op->far_row_max, op->oz_far_passes, op->ctx->stream);
+}
+
 bg_status ensure_work(bg_operator* op, int nrhs) {
   if (nrhs <= op->cap) return BG_OK;
   op->drop_graphs();  // the buffers below move
@@ -1500,8 +1618,9 @@ bg_status ensure_work(bg_operator* op, int nrhs) {
     BG_CHECK(op->w_y[l]->alloc(n), "work vectors");
     BG_CHECK(op->w_z[l]->alloc(n), "work vectors");
     // double-float split of y (complex: 16 columns at a time)
-    BG_CHECK(op->w_ydf[l]->alloc(op->cplx ? (size_t)op->nclusters(l) * op->np * op->np * 32 * sizeof(float2) : n),
-             "work vectors");
+    if (!op->far_oz || op->maxwell())
+      BG_CHECK(op->w_ydf[l]->alloc(op->cplx ? (size_t)op->nclusters(l) * op->np * op->np * 32 * sizeof(float2) : n),
+               "work vectors");
     const size_t tb = op->cplx ? far_h16c_btile_bytes(op->np * op->np) : far_h16_btile_bytes(op->np * op->np);
     if (op->maxwell()) {
       const size_t nv = (size_t)op->nclusters(l) * op->np * op->np * 4 * std::min(nrhs, (int)bg_operator::kMwRhsChunk) * sb;
@@ -1512,6 +1631,17 @@ bg_status ensure_work(bg_operator* op, int nrhs) {
       BG_CHECK(op->w_btiles[l]->alloc(tb * op->nclusters(l)), "work vectors");
       BG_CHECK(op->w_binv[l]->alloc(sizeof(float) * 32 * op->nclusters(l)), "work vectors");
     }
+  }
+  // digit panels of x for the FP64-accurate tensor-core products
+  {
+    op->oz_near_passes = oz_passes(op, op->dense.nrows, nrhs);
+    if (op->near_oz)
+      BG_CHECK(op->w_oz_near.alloc((size_t)op->dense.nrows * bsr_oz_panel_bytes(op->dense.B, op->cplx) * op->oz_near_passes),
+               "work vectors");
+    const int cols = op->maxwell() ? 4 * std::min(nrhs, (int)bg_operator::kMwRhsChunk) : nrhs;
+    op->oz_far_passes = oz_passes(op, op->n_far_work, cols);
+    if (op->far_oz) BG_CHECK(op->w_oz_far.alloc(oz_far_panels(op, nullptr) * op->oz_far_passes), "work vectors");
+    BG_CHECK(op->w_oz_fmax.alloc((size_t)2 * kOzMaxSegs * 32 * sizeof(int)), "work vectors");
   }
   if (op->fmm_fused) {
     // arrival counters of the fused upward pass: parents at levels
@@ -1561,7 +1691,7 @@ static void fill_fmm(const bg_operator* op, const void* fac, int kk, const void*
 // The product between T x and T^T y: superspace x in w_xss to superspace y in
 // w_yss, only on the operator's own work buffers (so it can be captured as a
 // CUDA graph and replayed).
-static bg_status apply_middle(bg_operator* op, int nrhs, int prec) {
+static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver) {
   cudaStream_t s = op->ctx->stream;
   const bool mixed = prec != BG_PREC_FP64;   // far field and transforms in FP32
   const bool near32 = prec == BG_PREC_FP32;  // near field in FP32 too
@@ -1582,9 +1712,14 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec) {
     const char* xs = static_cast<const char*>(near32 ? op->w_xss32.p : op->w_xss.p);
     char* ys = static_cast<char*>(near32 ? op->w_yss32.p : op->w_yss.p);
     for (int q = 0; q < nk; ++q) {
+      const bg_operator::KSlot& k = op->kslots[q];
+      if (!near32 && near_by_digits(op, k.dense_dig, nr, solver)) {
+        BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return oz_near_product(op, k.dense64, k.dense_dig, nrhs, q * nr, nr); }),
+                 "near-field product (batched wavenumbers, tensor cores)");
+        continue;
+      }
       BG_CHECK(cudaMemcpy2DAsync(op->kb_xs.p, nr * es, xs + (size_t)q * nr * es, (size_t)nrhs * es, nr * es, op->S,
                                  cudaMemcpyDeviceToDevice, s), "near-field column block");
-      const bg_operator::KSlot& k = op->kslots[q];
       BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] {
                  return near32 ? launch_bsr_fp32(true, op->dense.d_row_ptr.as<int>(), op->dense.d_col.as<int>(), k.dense32.p,
                                                  op->block_stride32(op->dense.B), op->dense.nrows, op->dense.B,
@@ -1602,16 +1737,12 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec) {
     BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return launch_bsr_fp32(op->cplx, op->dense.d_row_ptr.as<int>(), op->dense.d_col.as<int>(), op->d_dense32.p,
                         op->block_stride32(op->dense.B), op->dense.nrows, op->dense.B, op->w_xss32.p, op->w_yss32.p, nrhs, 0, s, pl.near_kernel); }),
              "near-field product (FP32)");
-  } else if (mixed && !op->cplx && op->d_oz_tiles.p && pl.mixed_near == 0) {
+  } else if ((!mixed || pl.mixed_near == 0) && near_by_digits(op, op->d_dense_dig, nrhs, solver)) {
     // FP64-accurate near field on the tensor cores: 8 integer digits of 7
     // bits per operand, exact integer accumulation, one rounding at the end
-    BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] {
-               return launch_near_oz(op->dense.d_row_ptr.as<int>(), op->dense.d_col.as<int>(), op->dense.nrows,
-                                     op->dense.B, op->d_oz_tiles.p, op->d_oz_rexp.as<int>(), op->w_xss.as<double>(),
-                                     op->S, nrhs, op->w_oz_panels.p, op->w_oz_fmax.as<int>(), op->w_yss.as<double>(),
-                                     nrhs, nrhs, op->d_err.as<int>(), s); }),
+    BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return oz_near_product(op, op->d_dense64, op->d_dense_dig, nrhs, 0, nrhs); }),
              "near-field product (tensor cores, integer digits)");
-  } else if (mixed && !op->cplx && op->d_dense_df.p) {
+  } else if (mixed && !op->cplx && op->d_dense_df.p && (pl.mixed_near != 0 || !op->near_oz)) {
     // FP64-accurate near field in double-float: blocks and x as FP32 (hi, lo)
     // pairs, exact products and compensated sums (about 1e-14 relative)
     BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_split_df(op->w_xss.p, ss_n, op->w_xss_df.p, s); }),
@@ -1848,7 +1979,33 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec) {
       }
       return BG_OK;
     };
-    for (int l = 0; l <= op->leaf_level && !tc && !tcc && !tcc_kb; ++l) {
+    // FP64 far field on the tensor cores, all levels in one launch
+    const bool oz_far = !mixed && op->far_oz && op->store_far && !(solver && op->maxwell());
+    if (oz_far && op->maxwell()) {
+      const std::complex<double> kap(op->kre, op->kim), mk2 = -1.0 / (kap * kap);
+      for (int r0 = 0; r0 < nrhs; r0 += bg_operator::kMwRhsChunk) {
+        const int nr = std::min((int)bg_operator::kMwRhsChunk, nrhs - r0);
+        for (int l = 0; l <= op->leaf_level; ++l)
+          BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_in(Sfar, op->nclusters(l), np2, op->w_y[l]->p, nrhs, r0,
+                                                                          nr, op->d_tan64[l]->p, op->w_yv[l]->p, s); }),
+                   "Maxwell far-field columns");
+        BG_CHECK(timed_launch(op->ctx, KC_FAR64, [&] { return oz_far_product(op, op->d_far_df, op->w_yv, op->w_zv, 4 * nr, 0, 4 * nr); }),
+                 "far-field product (tensor cores, integer digits)");
+        for (int l = 0; l <= op->leaf_level; ++l)
+          BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_out(Sfar, op->nclusters(l), np2, op->w_zv[l]->p, nrhs, r0,
+                                                                           nr, op->d_tan64[l]->p, mk2.real(), mk2.imag(),
+                                                                           op->w_z[l]->p, s); }),
+                   "Maxwell far-field columns");
+      }
+    } else if (oz_far) {
+      // batched wavenumbers: wavenumber q's couplings on column block q
+      const int nk = op->kbatched() ? (int)op->kslots.size() : 1, nr = nrhs / nk;
+      for (int q = 0; q < nk; ++q)
+        BG_CHECK(timed_launch(op->ctx, KC_FAR64, [&] { return oz_far_product(op, op->kbatched() ? op->kslots[q].far_df : op->d_far_df,
+                                                                     op->w_y, op->w_z, nrhs, q * nr, nr); }),
+                 "far-field product (tensor cores, integer digits)");
+    }
+    for (int l = 0; l <= op->leaf_level && !tc && !tcc && !tcc_kb && !oz_far; ++l) {
       const BsrSegment& f = op->far[l];
       if (f.col.empty()) {
         BG_CHECK(cudaMemsetAsync(op->w_z[l]->p, 0, (size_t)op->vd * op->nclusters(l) * op->R * nrhs * sfar, s),
@@ -1979,7 +2136,7 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec) {
 // to direct launches for this operator.
 // Batched wavenumbers: column block q of the row-major dof vectors (nrhs /
 // nslots columns) goes through slot q's operator.
-static bg_status apply_wavenumber_blocks(bg_operator* op, int nrhs, int prec, const void* xdof, void* ydof) {
+static bg_status apply_wavenumber_blocks(bg_operator* op, int nrhs, int prec, const void* xdof, void* ydof, bool solver) {
   const int nk = (int)op->kslots.size();
   if (nrhs % nk) return set_error(op->ctx, BG_INVALID_ARG, "batched wavenumbers: columns must be a multiple of the wavenumbers");
   const int nr = nrhs / nk;
@@ -1995,7 +2152,7 @@ static bg_status apply_wavenumber_blocks(bg_operator* op, int nrhs, int prec, co
     BG_CHECK(cudaMemcpy2DAsync(op->w_kx.p, nr * usz, static_cast<const char*>(xdof) + off, pitch, nr * usz, op->N,
                                cudaMemcpyDeviceToDevice, s), "wavenumber column block");
     op->activate_slot(q);
-    st = apply_operator(op, nr, prec, op->w_kx.p, op->w_ky.p);
+    st = apply_operator(op, nr, prec, op->w_kx.p, op->w_ky.p, solver);
     if (st == BG_OK)
       BG_CHECK(cudaMemcpy2DAsync(static_cast<char*>(ydof) + off, pitch, op->w_ky.p, nr * usz, nr * usz, op->N,
                                  cudaMemcpyDeviceToDevice, s), "wavenumber column block");
@@ -2018,9 +2175,9 @@ static bool kbatch_one_pass(const bg_operator* op, int prec) {
   return true;
 }
 
-bg_status apply_operator(bg_operator* op, int nrhs, int prec, const void* xdof, void* ydof) {
+bg_status apply_operator(bg_operator* op, int nrhs, int prec, const void* xdof, void* ydof, bool solver) {
   if (op->kbatched()) {
-    if (!kbatch_one_pass(op, prec)) return apply_wavenumber_blocks(op, nrhs, prec, xdof, ydof);
+    if (!kbatch_one_pass(op, prec)) return apply_wavenumber_blocks(op, nrhs, prec, xdof, ydof, solver);
     const int nk = (int)op->kslots.size();
     if (nrhs % nk)
       return set_error(op->ctx, BG_INVALID_ARG, "batched wavenumbers: columns must be a multiple of the wavenumbers");
@@ -2039,23 +2196,25 @@ bg_status apply_operator(bg_operator* op, int nrhs, int prec, const void* xdof, 
   bg_status st = BG_OK;
   bg_context* ctx = op->ctx;
   if (ctx->profiling || !op->use_graphs) {
-    st = apply_middle(op, nrhs, prec);
+    st = apply_middle(op, nrhs, prec, solver);
   } else {
-    // one graph per shape and wavenumber slot (the slots' fields differ)
-    const long key = bg_operator::plan_key(nrhs, prec) + ((long)(op->kslot_active + 1) << 40);
+    // one graph per shape, wavenumber slot (the slots' fields differ) and, for
+    // Maxwell, use (the solver's products take other kernels)
+    const long key = bg_operator::plan_key(nrhs, prec) + ((long)(op->kslot_active + 1) << 40) +
+                     (solver && op->maxwell() ? 1l << 60 : 0);
     auto it = op->graphs.find(key);
     if (it == op->graphs.end() && !op->graph_seen.count(key)) {
       // first product of this shape: direct launches (they also raise the
       // kernels' shared-memory limits, which a capture must not do)
       op->graph_seen.insert(key);
-      st = apply_middle(op, nrhs, prec);
+      st = apply_middle(op, nrhs, prec, solver);
     } else if (it == op->graphs.end()) {
       // capture: count the launches the graph holds, per kernel class
       const long l0 = ctx->launches;
       long c0[8];
       for (int c = 0; c < 8; ++c) c0[c] = ctx->class_launches[c];
       cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-      bg_status mst = e == cudaSuccess ? apply_middle(op, nrhs, prec) : BG_DEVICE_ERROR;
+      bg_status mst = e == cudaSuccess ? apply_middle(op, nrhs, prec, solver) : BG_DEVICE_ERROR;
       cudaGraph_t g = nullptr;
       if (e == cudaSuccess) e = cudaStreamEndCapture(s, &g);
       bg_operator::ProductGraph pg;
@@ -2069,7 +2228,7 @@ bg_status apply_operator(bg_operator* op, int nrhs, int prec, const void* xdof, 
       if (e != cudaSuccess || mst != BG_OK || !pg.exec) {
         if (pg.exec) cudaGraphExecDestroy(pg.exec);
         op->use_graphs = false;
-        st = apply_middle(op, nrhs, prec);
+        st = apply_middle(op, nrhs, prec, solver);
       } else {
         it = op->graphs.emplace(key, pg).first;
       }
@@ -2166,11 +2325,11 @@ extern "C" bg_status bg_operator_autotune(bg_operator* op, int nrhs, int precisi
   // which also raises the kernels' shared-memory limits)
   auto time_plan = [&](const bg_launch_plan& p, double* ms) -> bg_status {
     op->plans[key] = p;
-    bg_status r = apply_middle(op, nrhs, precision);
+    bg_status r = apply_middle(op, nrhs, precision, false);
     if (r != BG_OK) return r;
     BG_CHECK(cudaEventRecord(ev.a, s), "autotune events");
     for (int i = 0; i < reps; ++i)
-      if ((r = apply_middle(op, nrhs, precision)) != BG_OK) return r;
+      if ((r = apply_middle(op, nrhs, precision, false)) != BG_OK) return r;
     BG_CHECK(cudaEventRecord(ev.b, s), "autotune events");
     BG_CHECK(cudaEventSynchronize(ev.b), "autotune events");
     if ((r = check_device_flag(op)) != BG_OK) return r;

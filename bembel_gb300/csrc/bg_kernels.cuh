@@ -212,22 +212,50 @@ cudaError_t launch_bsr_df(const int* row_ptr, const int* col, const void* blocks
                           const void* x, void* y, int nrhs, int accumulate, cudaStream_t s);
 // out[t] = (hi, lo) of in[t] (FP64), t < n
 cudaError_t launch_split_df(const void* in, long n, void* out, cudaStream_t s);
-// FP64-accurate near field on the tensor cores (bg_near_tc.cu) for real
-// operators with leaf blocks of B = 4, 16 or 36 rows: oz_supported(B);
-// bytes of the digit tiles of nblocks blocks and of the x digit panels of
-// nclusters clusters; launch_oz_build turns the FP64 blocks (column-major,
-// stride bstride) into row exponents rexp [nrows * B] and digit tiles;
-// launch_near_oz writes y (rows of ldy entries, nrhs columns) = A x for x
-// FP64 [xrows][ldx], panels and fmax (32 ints) its scratch, err the bounded
-// waits' flag
-bool oz_supported(int B);
-size_t oz_tile_bytes(int B, long nblocks);
-size_t oz_panel_bytes(int B, long nclusters);
-cudaError_t launch_oz_build(const int* row_ptr, const double* blocks, long bstride, int nrows, int B, int* rexp,
-                            void* tiles, long nblocks, cudaStream_t s);
-cudaError_t launch_near_oz(const int* row_ptr, const int* col, int nrows, int B, const void* tiles,
-                           const int* rexp, const double* x, long xrows, int ldx, void* panels, int* fmax,
-                           double* y, int ldy, int nrhs, int* err, cudaStream_t s);
+// FP64-accurate block-sparse products on the tensor cores (bg_bsr_oz.cu):
+// real couplings as 8 digit bytes each, complex ones as FP32 (hi, lo) pairs (of
+// Re, then of Im) or FP64. A segment is one FMM level of the far field or the
+// near field; all segments of a launch share the block size and the storage.
+constexpr int kOzMaxSegs = kMaxFarLevels;
+struct OzSeg {
+  const int* row_ptr;
+  const int* col;
+  const unsigned char* tiles;  // block k at + k tstride bytes (pairs of Im: im_off bytes further)
+  long tstride, im_off;
+  const int* rexp;             // row exponents [rows][B]
+  const double* x;             // [ncl B][ldx] (complex interleaved)
+  double* y;                   // [rows B][ldx], written
+  unsigned char* panels;       // scratch, bsr_oz_panel_bytes per cluster and pass (those of pass p at + p pass_panels)
+  int ncl;                     // column clusters
+};
+struct OzArgs {
+  OzSeg seg[kOzMaxSegs];
+  int nseg;
+  const int2* work;    // (segment, row) of every block row; nullptr: all rows of segment 0
+  int nwork;
+  int B, ldx, c0, ncols;  // columns c0 .. c0 + ncols - 1 of rows of ldx scalars
+  size_t pass_panels;
+  int* fmax;           // scratch, 32 ints per segment and pass
+  int* err;
+  // set by the launcher
+  int nitems, unit, rg, nks, kw, nch, bps, nc, stages, raws, chunk_blocks;
+  uint32_t slice, stage, raw, raw_off, panel, tstride;
+};
+// max_row_blocks: the longest block row; pairs: complex blocks as FP32 pairs, not FP64
+bool bsr_oz_supported(int B, bool cplx, bool pairs, int max_row_blocks);
+size_t bsr_oz_panel_bytes(int B, bool cplx);  // 0: block size not supported
+long bsr_oz_tile_stride(int B);               // bytes between the (real) blocks' digit bytes
+// row exponents [nrows B] of FP64 blocks (column-major, complex interleaved), digit bytes of real ones
+cudaError_t launch_bsr_oz_rows(bool cplx, const int* row_ptr, const void* blocks, long bstride, int nrows, int B,
+                               int* rexp, cudaStream_t s);
+cudaError_t launch_bsr_oz_tiles(const int* row_ptr, const double* blocks, long bstride, int nrows, int B,
+                                const int* rexp, void* tiles, cudaStream_t s);
+// cplx: complex pairs (pairs set) or FP64, else digit bytes; max_row_blocks as
+// bsr_oz_supported, over the segments; max_passes: passes of 32 columns
+// (complex: 16) the panel scratch has room for
+cudaError_t launch_bsr_oz(bool cplx, bool pairs, OzArgs a, int max_row_blocks, int max_passes, cudaStream_t s);
+// digit bytes, one right-hand side (ldx 1) without panels, double-float: x_pairs the FP32 (hi, lo) pairs of x
+cudaError_t launch_digits_one(const OzSeg& g, const void* x_pairs, int nrows, int B, cudaStream_t s);
 // FP64-accurate near field of real operators for exactly 32 right-hand
 // sides (B <= 42): columns 0 .. 23 in double-float from the (hi, lo) pairs
 // and the split x, columns 24 .. 31 in FP64 from blocks64 and x64 (row-major

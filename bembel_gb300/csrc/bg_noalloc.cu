@@ -27,13 +27,14 @@
 // fully written before it is read, and the FP32 accumulator of the mixed path
 // is cleared with cudaMemsetAsync on each call.
 //
-// The FP64 far field follows bg_matvec: real operators multiply the
-// double-float (hi, lo) copies of the couplings when they exist, complex ones
-// the split real and imaginary pairs, and only operators without those copies
-// read the FP64 blocks. Operators assembled with keep_fp64_blocks = 0 (as the
-// serving cache builds them) have released the FP64 blocks and always take
-// the double-float route; an operator holding neither is refused with
-// BG_UNSUPPORTED before any device work.
+// The FP64 far field reads what bg_matvec reads: real operators the couplings'
+// digit bytes (in double-float arithmetic: the tensor-core product's digit
+// panels would not fit the array) or, where the block size has no digits,
+// their double-float (hi, lo) copies, complex ones the split real and imaginary
+// pairs, and only operators without those read the FP64 blocks. Operators
+// assembled with keep_fp64_blocks = 0 (as the serving cache builds them) have
+// released the FP64 blocks and always take the former route; an operator
+// holding neither is refused with BG_UNSUPPORTED before any device work.
 #include <cstdint>
 #include <mutex>
 
@@ -185,7 +186,12 @@ static bg_status product_in_scratch(bg_operator* op, bool mixed, const ScratchPl
                                   f.d_row_ptr.as<int>(), f.d_col.as<int>(), f.nrows, np2, (float)op->kre,
                                   (float)op->kim, Y(l), Z(l), 1, s),
                  "far-field product (FP32 fused)");
-      else if (op->d_far_df[l]->p && op->cplx) {
+      else if (op->far_digits() && op->d_far_df[l]->p) {
+        // the couplings' digit bytes, one right-hand side in double-float
+        NA_CHECK(launch_split_df(Y(l), (long)op->nclusters(l) * op->R, base + sp.ydf[l], s), "far-field split of Y");
+        NA_CHECK(launch_digits_one(oz_far_seg(op, l, nullptr, Z(l)), base + sp.ydf[l], f.nrows, f.B, s),
+                 "far-field product (digits)");
+      } else if (op->d_far_df[l]->p && op->cplx) {
         // Re K split(y) + Im K split(i y), the second pass accumulating
         const long sdf = ((long)f.B * f.B + 1) / 2 * 2;
         const float2* kr = op->d_far_df[l]->as<float2>();

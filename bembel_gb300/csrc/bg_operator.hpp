@@ -159,7 +159,7 @@ struct bg_operator {
   // swapping the slot's fields into the operator's (activate_slot).
   struct KSlot {
     double kre = 0.0, kim = 0.0;
-    DevBuf dense64, dense32;
+    DevBuf dense64, dense32, dense_dig;
     std::vector<DevBuf*> far64, far_df, atiles, ainv;
     bool far_tiles = false;
   };
@@ -180,6 +180,7 @@ struct bg_operator {
     std::swap(kim, k.kim);
     std::swap(d_dense64, k.dense64);
     std::swap(d_dense32, k.dense32);
+    std::swap(d_dense_dig, k.dense_dig);
     std::swap(d_far64, k.far64);
     std::swap(d_far_df, k.far_df);
     std::swap(d_far_atiles, k.atiles);
@@ -215,16 +216,26 @@ struct bg_operator {
   std::vector<DevBuf*> d_pts64, d_pts32, d_centres;  // per level
   std::vector<DevBuf*> d_tan64, d_tan32;             // per level, Maxwell: tangents dx, dy of every point
   DevBuf d_dense64;                       // dense blocks (FP64)
+  DevBuf d_dense_dig;                     // near_oz operators: their digit bytes (real; bg_bsr_oz.cu), then their
+                                          // row exponents
   DevBuf d_dense32;                       // FP32 copy of the dense blocks (BG_PREC_FP32)
   DevBuf d_dense_df;                      // real operators: FP32 (hi, lo) pairs of the dense blocks, the
                                           // near field of BG_PREC_MIXED products (double-float, FP64 accuracy)
-  // real operators, leaf blocks of 4, 16 or 36 rows: the near field as 8
-  // FP16 integer digits per entry in tensor-core tiles (bg_near_tc.cu), the
-  // exponent of every block-row row, and the per-product x digit panels and
-  // column exponents
-  DevBuf d_oz_tiles, d_oz_rexp, w_oz_panels, w_oz_fmax;
+  // FP64-accurate tensor-core products (bg_bsr_oz.cu): the digit panels of x
+  // (near field, far field; oz_near_passes / oz_far_passes panels per cluster)
+  // and column exponents, scratch of one product; the longest block rows
+  DevBuf w_oz_near, w_oz_far, w_oz_fmax;
+  int oz_near_passes = 0, oz_far_passes = 0;
+  int near_row_max = 0, far_row_max = 0;
   std::vector<DevBuf*> d_far64;           // per level
-  std::vector<DevBuf*> d_far_df;          // per level: FP32 (hi, lo) pairs of d_far64 (real operators)
+  std::vector<DevBuf*> d_far_df;          // per level: the couplings of the FP64-accurate products: 8 digit bytes
+                                          // each (far_digits), else FP32 (hi, lo) pairs (complex: of Re, then of
+                                          // Im); with far_oz the row exponents behind them
+  // FP64-accurate products on the tensor cores (bg_bsr_oz.cu) for the far and
+  // the near field, fixed by the block sizes and rows when the operator is
+  // created
+  bool far_oz = false, near_oz = false;
+  bool far_digits() const { return far_oz && !cplx; }
   std::vector<DevBuf*> d_far_atiles;      // per level: FP16 hi/lo tensor-core tiles of the low-rank blocks
   std::vector<DevBuf*> d_far_ainv;        // per level: inverse power-of-two scale of every tile
   bool far_tiles = false;                 // every far-field level has its tiles
@@ -318,6 +329,11 @@ struct bg_operator {
   long block_stride(int B) const { return cplx ? (long)B * B : ((long)B * B + 1) / 2 * 2; }
   // FP32 blocks: stride a multiple of 16 bytes
   long block_stride32(int B) const { return cplx ? ((long)B * B + 1) / 2 * 2 : ((long)B * B + 3) / 4 * 4; }
+  // bytes of the digits or pairs of nblocks blocks of size B, ahead of the row exponents
+  size_t digit_bytes(long nblocks, int B) const {
+    const long s = ((long)B * B + 1) / 2 * 2 * 8;
+    return (size_t)nblocks * s * (cplx ? 2 : 1);
+  }
   int stype(bool fp32) const { return (fp32 ? 2 : 0) + (cplx ? 1 : 0); }
   // Maxwell: the far field is stored as the scalar kernel matrix of each
   // cluster pair (np^2 x np^2) and applied to kMwRhsChunk right-hand sides at a time
@@ -328,6 +344,8 @@ struct bg_operator {
 
 bg_status set_error(bg_context* ctx, bg_status st, const std::string& msg);
 std::vector<double> basis3_table(int P, const bg::Rule1D& gr);
+// level l of the far field as a segment of bg_bsr_oz.cu (far_oz operators)
+bg::OzSeg oz_far_seg(const bg_operator* op, int l, const void* x, void* y);
 // child bookkeeping: a context is released only after its last child
 void context_retain(bg_context* ctx);
 void context_release(bg_context* ctx);
@@ -338,4 +356,10 @@ bg_status check_device_flag(bg_operator* op);
 // BG_PREC_FP64 the FP64 H2 matrix (stored far field); BG_PREC_MIXED FP64 near
 // field plus the FP32 fused far field (forward/backward transforms in FP32);
 // BG_PREC_FP32 as MIXED with the near field in FP32 as well.
-bg_status apply_operator(bg_operator* op, int nrhs, int prec, const void* xdof, void* ydof);
+// solver: a product inside bg_solve. Maxwell's keep the double-float far field
+// and the FP64-pipe near field there: its flexible GMRES with an FP32 inner
+// solve turns differences of 1e-16 in the products into differences of the
+// stopping residual's size in x (1.5e-9 of the field at a tolerance of 1e-8,
+// against 1e-10 for the scalar operators), and its solves are to stay
+// reproducible.
+bg_status apply_operator(bg_operator* op, int nrhs, int prec, const void* xdof, void* ydof, bool solver = false);

@@ -291,7 +291,7 @@ bg_status fgmres(Krylov& K, int prec, Krylov* inner, int inner_prec, double inne
       if (e != cudaSuccess) return cuda_status(op->ctx, e, "gmres");
       first_cycle = false;
     } else {
-      if ((st = apply_operator(op, k, prec, x, r.p)) != BG_OK) return st;
+      if ((st = apply_operator(op, k, prec, x, r.p, true)) != BG_OK) return st;
       ++(low ? cnt->mixed_mv : cnt->fp64_mv);
       timed_launch(op->ctx, KC_KRYLOV, [&] {
         k_residual<S><<<nblk(nk), 256, 0, s>>>(static_cast<const S*>(b), nk, r.as<S>());
@@ -347,7 +347,7 @@ bg_status fgmres(Krylov& K, int prec, Krylov* inner, int inner_prec, double inne
           cnt->inner_it += ic.outer_it;
           zj = zdst;
         }
-        if ((st = apply_operator(op, k, prec, zj, K.w.p)) != BG_OK) return st;
+        if ((st = apply_operator(op, k, prec, zj, K.w.p, true)) != BG_OK) return st;
         ++(low ? cnt->mixed_mv : cnt->fp64_mv);
         // classical Gram-Schmidt (gs_passes passes: two for the outer and the plain
         // FP64 solve, one for the inner preconditioning solve) and the norm, on the device;

@@ -307,13 +307,13 @@ typedef struct bg_launch_plan {
    * SMs, else 1); 1 one persistent CTA of four shared-memory stages per SM;
    * 2 two CTAs of two stages per SM. Results are identical. */
   int far_ctas;
-  /* FP64-accurate near field of BG_PREC_MIXED products of real operators:
-   * 0 built-in (the tensor-core product on 8 integer digits of 7 bits per
-   * operand, exact integer accumulation, where the leaf block size allows
-   * it: 4, 16 or 36 rows; else 1); 1 double-float on the FP32 pipes; 2 the
-   * double-float product with a quarter of 32 columns on the FP64 pipe
-   * (32 columns only, else 1). All agree with the FP64 product to about
-   * 1e-14 relative or better. */
+  /* FP64-accurate near field of BG_PREC_MIXED products: 0 built-in (the
+   * tensor-core product on 8 integer digits of 7 bits per operand, exact
+   * integer accumulation, which the FP64 product uses too, or for one or two
+   * columns the FP64 pipe); real operators also 1 double-float on the FP32
+   * pipes, 2 the double-float product with a quarter of 32 columns on the
+   * FP64 pipe (32 columns only, else 1). All agree with the FP64 product to
+   * about 1e-14 relative or better. */
   int mixed_near;
   /* couplings of the stored-tile far field of real operators (BG_PREC_MIXED,
    * BG_PREC_FP32): 0 built-in, the FP16 hi and lo tiles (three products per
