@@ -1685,6 +1685,7 @@ static void fill_fmm(const bg_operator* op, const void* fac, int kk, const void*
   f->Bq = op->Bq;
   f->L = op->leaf_level;
   f->kk = kk;
+  f->nc = 0;  // chosen by the launcher
 }
 
 // One H2 product on row-major FP64 work vectors (H2DenseProduct.hpp:33-165).

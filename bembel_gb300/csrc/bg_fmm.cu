@@ -31,9 +31,12 @@
 // the parent and applies the transposed moments, accumulating into the
 // superspace result.
 //
-// Layout: panels in shared memory are [row][32 columns], lane = column, so a
-// warp reads a row without bank conflicts and the 1-D factors are broadcast.
-// Warp w owns output rows w, w + 8, ... of every stage.
+// Layout: panels in shared memory are [row][nc columns], 32 columns or, for
+// FP64 products with fewer, the next power of two; a thread owns one column and
+// every nw-th output row of a stage. The FP64 pipe, which bounds these passes,
+// takes 64 cycles per warp instruction and SM quarter however few lanes have a
+// column, so few columns share their warps among output rows: one column
+// through 32-column panels costs as much as 32.
 #include <algorithm>
 #include <cstdint>
 #include <type_traits>
@@ -44,10 +47,18 @@ namespace bg {
 
 namespace {
 
-constexpr int kFmmThreads = 256;
-constexpr int kFmmWarps = kFmmThreads / 32;
+constexpr int kFmmThreads = 256, kFmmMaxThreads = 512;
 constexpr int kFmmCols = 32;
-constexpr int kMaxAcc = (kFmmMaxNp * kFmmMaxNp + kFmmWarps - 1) / kFmmWarps;
+constexpr int kFmmRows = kFmmThreads / kFmmCols;  // output rows at once, at least
+constexpr int kMaxAcc = (kFmmMaxNp * kFmmMaxNp + kFmmRows - 1) / kFmmRows;
+
+// Where a thread stands: column `lane` of the nc-column panel, and every nw-th
+// output row from w on
+struct FmmPos {
+  int w, lane, nw, nc;
+  __device__ __forceinline__ explicit FmmPos(int cols)
+      : w(threadIdx.x / cols), lane(threadIdx.x % cols), nw(blockDim.x / cols), nc(cols) {}
+};
 
 // son order (0,0), (1,0), (1,1), (0,1) (ElementTree.hpp:706-711): halves of child k
 __device__ __forceinline__ int half_s(int k) { return (k == 1 || k == 2) ? 1 : 0; }
@@ -61,7 +72,7 @@ struct FmmSmem {
   int* q_of;  // [w1][w1]: superspace row of the leaf cluster holding (a, b)
   T* X;    // [4 Bq][32] leaf inputs (up) / unused (down)
   T* W;    // [max(np w1, np^2)][32] stage scratch
-  T* V;    // [np^2][32] stage scratch
+  T* V;    // [max(np w1, np^2)][32] stage scratch
   T* C;    // [np^2][32] current child / leaf coefficients
   T* Zf;   // [np^2][32] (down) the parent's full coefficients
 };
@@ -70,27 +81,27 @@ template <typename T>
 __device__ __forceinline__ size_t align16(size_t n) { return (n * sizeof(T) + 15) / 16 * 16 / sizeof(T); }
 
 template <typename T>
-__device__ FmmSmem<T> carve(unsigned char* base, int np, int w1, int Bq, bool with_x) {
+__device__ FmmSmem<T> carve(unsigned char* base, int np, int w1, int Bq, int nc, bool with_x) {
   FmmSmem<T> s;
   const int np2 = np * np, wrows = max(np * w1, np2);
-  T* p = reinterpret_cast<T*>(base);
-  s.E = p;
-  p += align16<T>(2 * np2);
-  s.Ms = p;
-  p += align16<T>(np * w1);
-  s.Mt = p;
-  p += align16<T>(np * w1);
-  s.X = p;
-  if (with_x) p += (size_t)4 * Bq * kFmmCols;
-  s.W = p;
-  p += (size_t)wrows * kFmmCols;
-  s.V = p;
-  p += (size_t)np2 * kFmmCols;
-  s.C = p;
-  p += (size_t)np2 * kFmmCols;
-  s.Zf = p;
-  p += (size_t)np2 * kFmmCols;
-  s.q_of = reinterpret_cast<int*>(p);
+  T* at = reinterpret_cast<T*>(base);
+  s.E = at;
+  at += align16<T>(2 * np2);
+  s.Ms = at;
+  at += align16<T>(np * w1);
+  s.Mt = at;
+  at += align16<T>(np * w1);
+  s.X = at;
+  if (with_x) at += (size_t)4 * Bq * nc;
+  s.W = at;
+  at += (size_t)wrows * nc;
+  s.V = at;
+  at += (size_t)wrows * nc;
+  s.C = at;
+  at += (size_t)np2 * nc;
+  s.Zf = at;
+  at += (size_t)np2 * nc;
+  s.q_of = reinterpret_cast<int*>(at);
   return s;
 }
 
@@ -110,26 +121,26 @@ __device__ void load_factors(const FmmSmem<T>& s, const T* fac, const int* cmap,
 
 // V[cs][pt] = sum_ct Et[ct][pt] C[cs][ct]   (transfer up, stage 1, t direction)
 template <typename T>
-__device__ __forceinline__ void up_stage1(const T* Et, const T* C, T* V, int np, int w, int lane) {
+__device__ __forceinline__ void up_stage1(const T* Et, const T* C, T* V, int np, const FmmPos& p) {
   const int np2 = np * np;
-  for (int o = w; o < np2; o += kFmmWarps) {
+  for (int o = p.w; o < np2; o += p.nw) {
     const int cs = o / np, pt = o - cs * np;
     T acc = T(0);
-    for (int ct = 0; ct < np; ++ct) acc = fma(Et[ct * np + pt], C[(cs * np + ct) * kFmmCols + lane], acc);
-    V[o * kFmmCols + lane] = acc;
+    for (int ct = 0; ct < np; ++ct) acc = fma(Et[ct * np + pt], C[(cs * np + ct) * p.nc + p.lane], acc);
+    V[o * p.nc + p.lane] = acc;
   }
 }
 // acc[u] += sum_cs Es[cs][ps] V[cs][pt], output row o = w + 8u = ps np + pt
 template <typename T>
-__device__ __forceinline__ void up_stage2(const T* Es, const T* V, T* acc, int np, int w, int lane) {
+__device__ __forceinline__ void up_stage2(const T* Es, const T* V, T* acc, int np, const FmmPos& p) {
   const int np2 = np * np;
 #pragma unroll
   for (int u = 0; u < kMaxAcc; ++u) {
-    const int o = w + kFmmWarps * u;
+    const int o = p.w + p.nw * u;
     if (o < np2) {
       const int ps = o / np, pt = o - ps * np;
       T a = acc[u];
-      for (int cs = 0; cs < np; ++cs) a = fma(Es[cs * np + ps], V[(cs * np + pt) * kFmmCols + lane], a);
+      for (int cs = 0; cs < np; ++cs) a = fma(Es[cs * np + ps], V[(cs * np + pt) * p.nc + p.lane], a);
       acc[u] = a;
     }
   }
@@ -140,75 +151,75 @@ __device__ __forceinline__ void up_stage2(const T* Es, const T* V, T* acc, int n
 // other CTAs of this launch)
 template <typename T>
 __device__ void transfer_up_from_global(const FmmSmem<T>& s, const T* ychild, T* ypar, int par, int np, int kk,
-                                        int c0) {
-  const int np2 = np * np, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool on = c0 + lane < kk;
+                                        int c0, const FmmPos& p) {
+  const int np2 = np * np;
+  const bool on = c0 + p.lane < kk;
   T acc[kMaxAcc];
 #pragma unroll
   for (int u = 0; u < kMaxAcc; ++u) acc[u] = T(0);
   for (int k = 0; k < 4; ++k) {
-    const T* src = ychild + ((size_t)(4 * par + k) * np2) * kk + c0 + lane;
-    for (int o = w; o < np2; o += kFmmWarps) s.C[o * kFmmCols + lane] = on ? __ldcg(src + (size_t)o * kk) : T(0);
+    const T* src = ychild + ((size_t)(4 * par + k) * np2) * kk + c0 + p.lane;
+    for (int o = p.w; o < np2; o += p.nw) s.C[o * p.nc + p.lane] = on ? __ldcg(src + (size_t)o * kk) : T(0);
     __syncthreads();
-    up_stage1(s.E + half_t(k) * np2, s.C, s.V, np, w, lane);
+    up_stage1(s.E + half_t(k) * np2, s.C, s.V, np, p);
     __syncthreads();
-    up_stage2(s.E + half_s(k) * np2, s.V, acc, np, w, lane);
+    up_stage2(s.E + half_s(k) * np2, s.V, acc, np, p);
     __syncthreads();
   }
-  T* dst = ypar + ((size_t)par * np2) * kk + c0 + lane;
+  T* dst = ypar + ((size_t)par * np2) * kk + c0 + p.lane;
 #pragma unroll
   for (int u = 0; u < kMaxAcc; ++u) {
-    const int o = w + kFmmWarps * u;
+    const int o = p.w + p.nw * u;
     if (o < np2 && on) dst[(size_t)o * kk] = acc[u];
   }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kFmmThreads) k_fmm_up(FmmLevels<T> a) {
+__global__ void __launch_bounds__(kFmmMaxThreads) k_fmm_up(FmmLevels<T> a) {
   extern __shared__ __align__(16) unsigned char fmm_smem[];
   const int np = a.np, np2 = np * np, w1 = a.w1, Bq = a.Bq, kk = a.kk;
-  const FmmSmem<T> s = carve<T>(fmm_smem, np, w1, Bq, true);
-  const int P = blockIdx.x, chunk = blockIdx.y, c0 = chunk * kFmmCols;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool on = c0 + lane < kk;
+  const FmmSmem<T> s = carve<T>(fmm_smem, np, w1, Bq, a.nc, true);
+  const FmmPos p(a.nc);
+  const int P = blockIdx.x, chunk = blockIdx.y, c0 = chunk * a.nc;
+  const bool on = c0 + p.lane < kk;
   const int L = a.L;
   load_factors(s, a.fac, a.cmap, np, w1, Bq);
   // the 4 leaf clusters' superspace panels
-  for (int r = w; r < 4 * Bq; r += kFmmWarps)
-    s.X[r * kFmmCols + lane] = on ? a.x[((size_t)4 * P * Bq + r) * kk + c0 + lane] : T(0);
+  for (int r = p.w; r < 4 * Bq; r += p.nw)
+    s.X[r * p.nc + p.lane] = on ? a.x[((size_t)4 * P * Bq + r) * kk + c0 + p.lane] : T(0);
   __syncthreads();
   T acc[kMaxAcc];
 #pragma unroll
   for (int u = 0; u < kMaxAcc; ++u) acc[u] = T(0);
   for (int j = 0; j < 4; ++j) {
-    const T* Xj = s.X + (size_t)j * Bq * kFmmCols;
+    const T* Xj = s.X + (size_t)j * Bq * p.nc;
     // moments, s direction: W[i][b] = sum_a Ms[i][a] X[q(a, b)]
-    for (int o = w; o < np * w1; o += kFmmWarps) {
+    for (int o = p.w; o < np * w1; o += p.nw) {
       const int i = o / w1, b = o - i * w1;
       T v = T(0);
-      for (int aa = 0; aa < w1; ++aa) v = fma(s.Ms[i * w1 + aa], Xj[s.q_of[aa * w1 + b] * kFmmCols + lane], v);
-      s.W[o * kFmmCols + lane] = v;
+      for (int aa = 0; aa < w1; ++aa) v = fma(s.Ms[i * w1 + aa], Xj[s.q_of[aa * w1 + b] * p.nc + p.lane], v);
+      s.W[o * p.nc + p.lane] = v;
     }
     __syncthreads();
     // moments, t direction: C[i][i2] = sum_b W[i][b] Mt[i2][b]; written out as Y_L
-    T* yl = a.y[L] + ((size_t)(4 * P + j) * np2) * kk + c0 + lane;
-    for (int o = w; o < np2; o += kFmmWarps) {
+    T* yl = a.y[L] + ((size_t)(4 * P + j) * np2) * kk + c0 + p.lane;
+    for (int o = p.w; o < np2; o += p.nw) {
       const int i = o / np, i2 = o - i * np;
       T v = T(0);
-      for (int b = 0; b < w1; ++b) v = fma(s.W[(i * w1 + b) * kFmmCols + lane], s.Mt[i2 * w1 + b], v);
-      s.C[o * kFmmCols + lane] = v;
+      for (int b = 0; b < w1; ++b) v = fma(s.W[(i * w1 + b) * p.nc + p.lane], s.Mt[i2 * w1 + b], v);
+      s.C[o * p.nc + p.lane] = v;
       if (on) yl[(size_t)o * kk] = v;
     }
     __syncthreads();
-    up_stage1(s.E + half_t(j) * np2, s.C, s.V, np, w, lane);
+    up_stage1(s.E + half_t(j) * np2, s.C, s.V, np, p);
     __syncthreads();
-    up_stage2(s.E + half_s(j) * np2, s.V, acc, np, w, lane);
+    up_stage2(s.E + half_s(j) * np2, s.V, acc, np, p);
   }
   {
-    T* dst = a.y[L - 1] + ((size_t)P * np2) * kk + c0 + lane;
+    T* dst = a.y[L - 1] + ((size_t)P * np2) * kk + c0 + p.lane;
 #pragma unroll
     for (int u = 0; u < kMaxAcc; ++u) {
-      const int o = w + kFmmWarps * u;
+      const int o = p.w + p.nw * u;
       if (o < np2 && on) dst[(size_t)o * kk] = acc[u];
     }
   }
@@ -230,81 +241,79 @@ __global__ void __launch_bounds__(kFmmThreads) k_fmm_up(FmmLevels<T> a) {
     __syncthreads();
     if (!last) return;
     cur >>= 2;
-    transfer_up_from_global(s, a.y[l + 1], a.y[l], cur, np, kk, c0);
+    transfer_up_from_global(s, a.y[l + 1], a.y[l], cur, np, kk, c0, p);
   }
 }
 
 // W[ps][ct] = sum_pt Et[ct][pt] Z[ps][pt]   (transposed transfer, t direction)
 template <typename T>
-__device__ __forceinline__ void down_stage1(const T* Et, const T* Z, T* W, int np, int w, int lane) {
+__device__ __forceinline__ void down_stage1(const T* Et, const T* Z, T* W, int np, const FmmPos& p) {
   const int np2 = np * np;
-  for (int o = w; o < np2; o += kFmmWarps) {
+  for (int o = p.w; o < np2; o += p.nw) {
     const int ps = o / np, ct = o - ps * np;
     T v = T(0);
-    for (int pt = 0; pt < np; ++pt) v = fma(Et[ct * np + pt], Z[(ps * np + pt) * kFmmCols + lane], v);
-    W[o * kFmmCols + lane] = v;
+    for (int pt = 0; pt < np; ++pt) v = fma(Et[ct * np + pt], Z[(ps * np + pt) * p.nc + p.lane], v);
+    W[o * p.nc + p.lane] = v;
   }
 }
 // out[cs][ct] = base[cs][ct] + sum_ps Es[cs][ps] W[ps][ct]  (s direction);
 // base read from global (this level's far-field result)
 template <typename T>
 __device__ __forceinline__ void down_stage2(const T* Es, const T* W, const T* base, int kk, bool on, T* out, int np,
-                                            int w, int lane) {
+                                            const FmmPos& p) {
   const int np2 = np * np;
-  for (int o = w; o < np2; o += kFmmWarps) {
+  for (int o = p.w; o < np2; o += p.nw) {
     const int cs = o / np, ct = o - cs * np;
     T v = on ? base[(size_t)o * kk] : T(0);
-    for (int ps = 0; ps < np; ++ps) v = fma(Es[cs * np + ps], W[(ps * np + ct) * kFmmCols + lane], v);
-    out[o * kFmmCols + lane] = v;
+    for (int ps = 0; ps < np; ++ps) v = fma(Es[cs * np + ps], W[(ps * np + ct) * p.nc + p.lane], v);
+    out[o * p.nc + p.lane] = v;
   }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kFmmThreads) k_fmm_down(FmmLevels<T> a) {
+__global__ void __launch_bounds__(kFmmMaxThreads) k_fmm_down(FmmLevels<T> a) {
   extern __shared__ __align__(16) unsigned char fmm_smem[];
   const int np = a.np, np2 = np * np, w1 = a.w1, Bq = a.Bq, kk = a.kk;
-  const FmmSmem<T> s = carve<T>(fmm_smem, np, w1, Bq, false);
-  const int P = blockIdx.x, c0 = blockIdx.y * kFmmCols;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool on = c0 + lane < kk;
+  const FmmSmem<T> s = carve<T>(fmm_smem, np, w1, Bq, a.nc, false);
+  const FmmPos p(a.nc);
+  const int P = blockIdx.x, c0 = blockIdx.y * a.nc;
+  const bool on = c0 + p.lane < kk;
   const int L = a.L;
   load_factors(s, a.fac, a.cmap, np, w1, Bq);
   // full coefficients of the level-0 ancestor: its far-field result
   {
-    const T* z0 = a.z[0] + ((size_t)(P >> (2 * (L - 1))) * np2) * kk + c0 + lane;
-    for (int o = w; o < np2; o += kFmmWarps) s.Zf[o * kFmmCols + lane] = on ? z0[(size_t)o * kk] : T(0);
+    const T* z0 = a.z[0] + ((size_t)(P >> (2 * (L - 1))) * np2) * kk + c0 + p.lane;
+    for (int o = p.w; o < np2; o += p.nw) s.Zf[o * p.nc + p.lane] = on ? z0[(size_t)o * kk] : T(0);
   }
   __syncthreads();
   // down the ancestor path to the parent P at level L - 1
   for (int l = 1; l <= L - 1; ++l) {
     const int al = P >> (2 * (L - 1 - l)), k = al & 3;
-    down_stage1(s.E + half_t(k) * np2, s.Zf, s.W, np, w, lane);
+    down_stage1(s.E + half_t(k) * np2, s.Zf, s.W, np, p);
     __syncthreads();
-    down_stage2(s.E + half_s(k) * np2, s.W, a.z[l] + ((size_t)al * np2) * kk + c0 + lane, kk, on, s.Zf, np, w,
-                lane);
+    down_stage2(s.E + half_s(k) * np2, s.W, a.z[l] + ((size_t)al * np2) * kk + c0 + p.lane, kk, on, s.Zf, np, p);
     __syncthreads();
   }
   for (int j = 0; j < 4; ++j) {
     const int leaf = 4 * P + j;
-    down_stage1(s.E + half_t(j) * np2, s.Zf, s.W, np, w, lane);
+    down_stage1(s.E + half_t(j) * np2, s.Zf, s.W, np, p);
     __syncthreads();
-    down_stage2(s.E + half_s(j) * np2, s.W, a.z[L] + ((size_t)leaf * np2) * kk + c0 + lane, kk, on, s.C, np, w,
-                lane);
+    down_stage2(s.E + half_s(j) * np2, s.W, a.z[L] + ((size_t)leaf * np2) * kk + c0 + p.lane, kk, on, s.C, np, p);
     __syncthreads();
     // transposed moments, t direction: V[i][b] = sum_j Mt[j][b] C[i][j]
-    for (int o = w; o < np * w1; o += kFmmWarps) {
+    for (int o = p.w; o < np * w1; o += p.nw) {
       const int i = o / w1, b = o - i * w1;
       T v = T(0);
-      for (int jj = 0; jj < np; ++jj) v = fma(s.Mt[jj * w1 + b], s.C[(i * np + jj) * kFmmCols + lane], v);
-      s.V[o * kFmmCols + lane] = v;
+      for (int jj = 0; jj < np; ++jj) v = fma(s.Mt[jj * w1 + b], s.C[(i * np + jj) * p.nc + p.lane], v);
+      s.V[o * p.nc + p.lane] = v;
     }
     __syncthreads();
     // s direction: y[q(a, b)] += sum_i Ms[i][a] V[i][b]
-    T* yo = a.out + ((size_t)leaf * Bq) * kk + c0 + lane;
-    for (int o = w; o < w1 * w1; o += kFmmWarps) {
+    T* yo = a.out + ((size_t)leaf * Bq) * kk + c0 + p.lane;
+    for (int o = p.w; o < w1 * w1; o += p.nw) {
       const int aa = o / w1, b = o - aa * w1;
       T v = T(0);
-      for (int i = 0; i < np; ++i) v = fma(s.Ms[i * w1 + aa], s.V[(i * w1 + b) * kFmmCols + lane], v);
+      for (int i = 0; i < np; ++i) v = fma(s.Ms[i * w1 + aa], s.V[(i * w1 + b) * p.nc + p.lane], v);
       if (on) {
         T* dst = yo + (size_t)s.q_of[o] * kk;
         *dst += v;
@@ -642,34 +651,50 @@ cudaError_t fmm_launch_t(bool up, const FmmLevels<T>& a, const double* hfac, int
 }
 
 template <typename T>
-size_t fmm_smem_bytes(int np, int w1, int Bq, bool with_x) {
+size_t fmm_smem_bytes(int np, int w1, int Bq, int nc, bool with_x) {
   auto a16 = [](size_t n) { return (n * sizeof(T) + 15) / 16 * 16; };
   const int np2 = np * np, wrows = std::max(np * w1, np2);
   return a16(2 * np2) + 2 * a16(np * w1) +
-         sizeof(T) * kFmmCols * ((with_x ? (size_t)4 * Bq : 0) + wrows + 3 * (size_t)np2) +
+         sizeof(T) * nc * ((with_x ? (size_t)4 * Bq : 0) + 2 * (size_t)wrows + 2 * (size_t)np2) +
          sizeof(int) * (size_t)w1 * w1;
 }
 
 template <typename T>
-cudaError_t fmm_launch(bool up, const FmmLevels<T>& a, const double* hfac, int nparents, cudaStream_t s) {
+cudaError_t fmm_launch(bool up, FmmLevels<T> a, const double* hfac, int nparents, cudaStream_t s) {
   if (nparents == 0 || a.kk == 0) return cudaSuccess;
   if (a.L < 1 || a.L >= kMaxFarLevels || a.np < 2 || a.np > kFmmMaxNp || a.w1 < 1 || a.w1 * a.w1 != a.Bq ||
       a.w1 > 16)
     return cudaErrorInvalidValue;
-  // compiled sizes: n_p 6, 9, 10 with P = 1, 2 (w1 = 4, 6)
-  if (hfac) {
+  // FP64 products of up to 16 columns: panels as wide as the columns there
+  // are, a thread per output row and column (the same sums in the same order).
+  // Both passes, 32-column panels of the compiled sizes -> this: P = 2, M = 4
+  // (n_p 9) 338 -> 73 us for one column, 338 -> 198 for 16; M = 5 890
+  // -> 91 and 452; M = 3, P = 1 (n_p 6) 94 -> 43 and 75. From 17 columns the
+  // panels are full and the compiled sizes are the faster. FP32 has 64 lanes a
+  // clock for the same work and is bound by latency, not by the pipe: 32-column
+  // panels for any number of columns.
+  a.nc = kFmmCols;
+  if (sizeof(T) == 8)
+    while (a.nc > 1 && a.nc / 2 >= a.kk) a.nc /= 2;
+  // compiled sizes: n_p 6 .. 10 with P = 1, 2 (w1 = 4, 6). Both passes at run
+  // time sizes -> compiled, 32 columns: n_p 8, M = 5, P = 1, FP32 229 -> 53 us,
+  // FP64 612 -> 581; n_p 7, complex, M = 2, P = 1, FP32 75 -> 20, FP64 115 -> 92
+  if (hfac && a.nc == kFmmCols) {
 #define BG_FMM_T(NPV, W1V) \
   if (a.np == NPV && a.w1 == W1V) return fmm_launch_t<T, NPV, W1V>(up, a, hfac, nparents, s);
-    BG_FMM_T(6, 4) BG_FMM_T(6, 6) BG_FMM_T(9, 4) BG_FMM_T(9, 6) BG_FMM_T(10, 4) BG_FMM_T(10, 6)
+    BG_FMM_T(6, 4) BG_FMM_T(6, 6) BG_FMM_T(7, 4) BG_FMM_T(7, 6) BG_FMM_T(8, 4)
+    BG_FMM_T(8, 6) BG_FMM_T(9, 4) BG_FMM_T(9, 6) BG_FMM_T(10, 4) BG_FMM_T(10, 6)
 #undef BG_FMM_T
   }
-  const size_t smem = fmm_smem_bytes<T>(a.np, a.w1, a.Bq, up);
+  const size_t smem = fmm_smem_bytes<T>(a.np, a.w1, a.Bq, a.nc, up);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
   auto kf = up ? k_fmm_up<T> : k_fmm_down<T>;
   cudaError_t e = smem_limit(kf, smem);
   if (e != cudaSuccess) return e;
-  const dim3 grid(nparents, (a.kk + kFmmCols - 1) / kFmmCols);
-  kf<<<grid, kFmmThreads, smem, s>>>(a);
+  const dim3 grid(nparents, (a.kk + a.nc - 1) / a.nc);
+  const int rows_threads = std::min(kFmmMaxThreads, (a.np * a.np * a.nc + 31) / 32 * 32);
+  const int threads = a.nc == kFmmCols ? kFmmThreads : std::max(a.nc * kFmmRows, rows_threads);
+  kf<<<grid, threads, smem, s>>>(a);
   return cudaGetLastError();
 }
 

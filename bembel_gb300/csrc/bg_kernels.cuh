@@ -295,6 +295,7 @@ struct FmmLevels {
   long cnt_off[kMaxFarLevels];
   long cnt_stride;
   int np, w1, Bq, L, kk;
+  int nc;  // columns per panel, set by the launcher
 };
 struct FmmLevelsAny {
   FmmLevels<double> f64;

@@ -116,3 +116,24 @@ def test_digit_products_keep_infinities_apart(ctx, kind):
     y = A.matvec(x)
     assert not np.isfinite(y[:, [2, 4]]).all(axis=0).any()
     assert np.isnan(y[:, 4]).any() and np.array_equal(y[:, [0, 1, 3, 5]], clean[:, [0, 1, 3, 5]])
+
+
+@pytest.mark.parametrize("P,np_", [(1, 6), (2, 6), (1, 7), (2, 8), (2, 9), (1, 10), (1, 11)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_fused_transforms_for_few_columns(ctx, P, np_, kind):
+    """The fused FP64 transforms pack the columns there are into a warp (1, 2,
+    4, .. 32 lanes a row): the product of any number of columns equals the
+    same columns of a 33-column product to rounding (1e-13, the transforms'
+    sums are the same ones), and the batched-GEMM transforms to 1e-12."""
+    d = _operator(ctx, SPHERE, 3, P, kind, 2.0, np_)
+    A = d.get_discrete_operator()
+    rng = np.random.default_rng(10)
+    x = rng.normal(size=(d.N, 33)) + (1j * rng.normal(size=(d.N, 33)) if kind else 0)
+    full = A.matvec(x)
+    for n in (1, 2, 3, 5, 9, 16, 17, 32):
+        y = A.matvec(x[:, :n])
+        assert np.linalg.norm(y - full[:, :n]) < 1e-13 * np.linalg.norm(full[:, :n]), n
+        d.set_plan(n, "fp64", transforms=1)
+        z = A.matvec(x[:, :n])
+        d.set_plan(n, "fp64")
+        assert np.linalg.norm(z - y) < 1e-12 * np.linalg.norm(y), n
