@@ -30,35 +30,49 @@ __device__ inline cd sub(cd a, cd b) { return a - b; }
 __device__ inline double addv(double a, double b) { return a + b; }
 __device__ inline cd addv(cd a, cd b) { return a + b; }
 
-// out[i][c] = sum_n conj(V[i][n][c]) w[n][c] for i < nv (one CTA per i)
-// (any k: with more columns than threads each thread sums whole columns)
+// The sums of the Krylov basis. Small ones are bound by the latency of their
+// chains, so a chain loads kAhead terms before it adds them, in the same fixed
+// order; large ones by reading the basis. Before -> after, per launch: column
+// norms of 32 columns, N = 6936, 298 -> 90 us (one CTA had all columns); one
+// column, N = 600: dots 14.6 -> 4.7 us (idle groups are not summed any more),
+// updates 11.3 -> 8.3. The sums also write the host's pinned copy (three
+// copies a step before) and the inverse norms (a launch). Dots and updates of 32
+// columns stay at 21 and 20 us: the basis once through memory.
+constexpr int kAhead = 8;
+
+// acc + conj(v[n]) w[n] over n = n0, n0 + step, .. < n1, in that order
 template <typename S>
-__global__ void k_mdot(const S* __restrict__ V, long vstride, const S* __restrict__ w, int N, int k, S* __restrict__ out) {
-  __shared__ S red[256];
-  const int i = blockIdx.x;
-  const int kp = k;  // columns
-  if (kp > (int)blockDim.x) {
-    const S* v = V + (long)i * vstride;
-    for (int c = threadIdx.x; c < kp; c += blockDim.x) {
-      S acc = zero<S>();
-      for (int n = 0; n < N; ++n) acc = addv(acc, conj_mul(v[(long)n * k + c], w[(long)n * k + c]));
-      out[(long)i * k + c] = acc;
-    }
-    return;
-  }
-  const int groups = blockDim.x / kp;
-  const int c = threadIdx.x % kp, g = threadIdx.x / kp;
+__device__ __forceinline__ S dot_chain(const S* __restrict__ v, const S* __restrict__ w, int n0, int n1, int step,
+                                       int k) {
   S acc = zero<S>();
-  if (g < groups) {
-    const S* v = V + (long)i * vstride;
-    for (int n = g; n < N; n += groups) acc = addv(acc, conj_mul(v[(long)n * k + c], w[(long)n * k + c]));
+  int n = n0;
+  for (; n + (kAhead - 1) * step < n1; n += kAhead * step) {
+    S a[kAhead], b[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      a[u] = v[(long)(n + u * step) * k];
+      b[u] = w[(long)(n + u * step) * k];
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) acc = addv(acc, conj_mul(a[u], b[u]));
   }
-  red[threadIdx.x] = acc;
+  for (; n < n1; n += step) acc = addv(acc, conj_mul(v[(long)n * k], w[(long)n * k]));
+  return acc;
+}
+
+// out[c] = sum_n conj(w[n][c]) w[n][c]: `groups` interleaved chains per column,
+// summed in order; a CTA holds cw columns (groups cw threads)
+template <typename S>
+__global__ void k_mdot(const S* __restrict__ w, int N, int k, int groups, int cw, S* __restrict__ out) {
+  __shared__ S red[256];
+  const int cl = threadIdx.x % cw, g = threadIdx.x / cw, c = blockIdx.x * cw + cl;
+  red[threadIdx.x] = c < k ? dot_chain<S>(w + c, w + c, g, N, groups, k) : zero<S>();
   __syncthreads();
-  if (threadIdx.x < kp) {
+  if (g == 0 && c < k) {
     S s = zero<S>();
-    for (int gg = 0; gg < groups; ++gg) s = addv(s, red[gg * kp + threadIdx.x]);
-    out[(long)i * k + threadIdx.x] = s;
+#pragma unroll 8
+    for (int gg = 0; gg < groups; ++gg) s = addv(s, red[gg * cw + cl]);
+    out[c] = s;
   }
 }
 // Blocked dot products for many vectors at once: CTA (i, chunk) reduces rows
@@ -70,63 +84,78 @@ __global__ void k_mdot_part(const S* __restrict__ V, long vstride, const S* __re
   __shared__ S red[256];
   const int i = blockIdx.x, ch = blockIdx.y, nch = gridDim.y;
   const int n0 = ch * rows_per, n1 = min(N, n0 + rows_per);
+  const S* v = V + (long)i * vstride;
+  S* to = part + ((long)i * nch + ch) * k;
   if (k > (int)blockDim.x) {  // more columns than threads: each thread sums whole columns of the chunk
-    const S* v = V + (long)i * vstride;
-    for (int c = threadIdx.x; c < k; c += blockDim.x) {
-      S acc = zero<S>();
-      for (int n = n0; n < n1; ++n) acc = addv(acc, conj_mul(v[(long)n * k + c], w[(long)n * k + c]));
-      part[((long)i * nch + ch) * k + c] = acc;
-    }
+    for (int c = threadIdx.x; c < k; c += blockDim.x) to[c] = dot_chain<S>(v + c, w + c, n0, n1, 1, k);
     return;
   }
-  const int groups = blockDim.x / k;
+  const int groups = min((int)blockDim.x / k, max(n1 - n0, 0));  // those with a row
   const int c = threadIdx.x % k, g = threadIdx.x / k;
-  S acc = zero<S>();
-  if (g < groups) {
-    const S* v = V + (long)i * vstride;
-    for (int n = n0 + g; n < n1; n += groups) acc = addv(acc, conj_mul(v[(long)n * k + c], w[(long)n * k + c]));
-  }
-  red[threadIdx.x] = acc;
+  if (g < groups) red[threadIdx.x] = dot_chain<S>(v + c, w + c, n0 + g, n1, blockDim.x / k, k);
   __syncthreads();
   if (threadIdx.x < k) {
     S s2 = zero<S>();
+#pragma unroll 8
     for (int gg = 0; gg < groups; ++gg) s2 = addv(s2, red[gg * k + threadIdx.x]);
-    part[((long)i * nch + ch) * k + threadIdx.x] = s2;
+    to[threadIdx.x] = s2;
   }
 }
+// 1 / sqrt(|d|) of a column's product with itself, 0 for 0
+__device__ inline double inv_norm(double d) { return d > 0 ? 1.0 / sqrt(d) : 0.0; }
+__device__ inline double inv_norm(cd d) { return d.re > 0 ? 1.0 / sqrt(d.re) : 0.0; }
+// The chunks' sums, to the device and to the host's pinned slot; with inv,
+// also the inverse column norms (nv = 1, the Gram column of w with itself)
 template <typename S>
-__global__ void k_reduce_parts(const S* __restrict__ part, int nv, int nch, int k, S* __restrict__ out) {
+__global__ void k_reduce_parts(const S* __restrict__ part, int nv, int nch, int k, S* __restrict__ out,
+                               S* __restrict__ host, double* __restrict__ inv) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nv * k) return;
   const int i = t / k, c = t % k;
+  const S* p = part + (long)i * nch * k + c;
   S s2 = zero<S>();
-  for (int ch = 0; ch < nch; ++ch) s2 = addv(s2, part[((long)i * nch + ch) * k + c]);
-  out[(long)i * k + c] = s2;
+  int ch = 0;
+  for (; ch + 2 * kAhead <= nch; ch += 2 * kAhead) {
+    S a[2 * kAhead];
+#pragma unroll
+    for (int u = 0; u < 2 * kAhead; ++u) a[u] = p[(long)(ch + u) * k];
+#pragma unroll
+    for (int u = 0; u < 2 * kAhead; ++u) s2 = addv(s2, a[u]);
+  }
+  for (; ch < nch; ++ch) s2 = addv(s2, p[(long)ch * k]);
+  out[t] = s2;
+  host[t] = s2;
+  if (inv) inv[c] = inv_norm(s2);
 }
 
-// w[n][c] -= sum_{i<nv} V[i][n][c] h[i][c]
-template <typename S>
-__global__ void k_vupdate(const S* __restrict__ V, long vstride, int nv, const S* __restrict__ h, int N, int k,
-                          S* __restrict__ w) {
+// x[n][c] -+ sum_{i<nv} V[i][n][c] h[i][c]
+template <typename S, bool SUB>
+__device__ __forceinline__ void combine(const S* __restrict__ V, long vstride, int nv, const S* __restrict__ h, int N,
+                                        int k, S* __restrict__ x) {
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long)N * k) return;
-  const int c = (int)(t % k);
-  S acc = w[t];
-  for (int i = 0; i < nv; ++i) acc = sub(acc, V[(long)i * vstride + t] * h[(long)i * k + c]);
-  w[t] = acc;
+  const S* v = V + t;
+  h += t % k;
+  S acc = x[t];
+  for (int i = 0; i < nv; i += kAhead) {
+    S a[kAhead], b[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int r = min(i + u, nv - 1);
+      a[u] = v[(long)r * vstride];
+      b[u] = h[(long)r * k];
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (i + u < nv) acc = SUB ? sub(acc, a[u] * b[u]) : addv(acc, a[u] * b[u]);
+  }
+  x[t] = acc;
 }
-// inv[c] = 1 / sqrt(|d[c]|) (0 when d[c] == 0), from a Gram column of w with itself
+// w[n][c] -= sum_{i<nv} V[i][n][c] h[i][c]
 template <typename S>
-__global__ void k_inv_norm(const S* __restrict__ d, int k, double* __restrict__ inv);
-template <>
-__global__ void k_inv_norm<double>(const double* __restrict__ d, int k, double* __restrict__ inv) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < k) inv[c] = d[c] > 0 ? 1.0 / sqrt(d[c]) : 0.0;
-}
-template <>
-__global__ void k_inv_norm<cd>(const cd* __restrict__ d, int k, double* __restrict__ inv) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < k) inv[c] = d[c].re > 0 ? 1.0 / sqrt(d[c].re) : 0.0;
+__global__ void __launch_bounds__(256, 3) k_vupdate(const S* __restrict__ V, long vstride, int nv, const S* __restrict__ h, int N, int k,
+                          S* __restrict__ w) {
+  combine<S, true>(V, vstride, nv, h, N, k, w);
 }
 // V_next[n][c] = w[n][c] * inv[c]
 template <typename S>
@@ -137,14 +166,9 @@ __global__ void k_vscale(const S* __restrict__ w, const double* __restrict__ inv
 }
 // x[n][c] += sum_i V[i][n][c] y[i][c]
 template <typename S>
-__global__ void k_xupdate(const S* __restrict__ V, long vstride, int nv, const S* __restrict__ y, int N, int k,
+__global__ void __launch_bounds__(256, 3) k_xupdate(const S* __restrict__ V, long vstride, int nv, const S* __restrict__ y, int N, int k,
                           S* __restrict__ x) {
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long)N * k) return;
-  const int c = (int)(t % k);
-  S acc = x[t];
-  for (int i = 0; i < nv; ++i) acc = addv(acc, V[(long)i * vstride + t] * y[(long)i * k + c]);
-  x[t] = acc;
+  combine<S, false>(V, vstride, nv, y, N, k, x);
 }
 // r = b - r (in place on r)
 template <typename S>
@@ -242,8 +266,10 @@ inline std::complex<double> cj(std::complex<double> v) { return std::conj(v); }
 template <typename S>
 bg_status col_norms(Krylov& K, const void* x, std::vector<double>* out) {
   cudaStream_t s = K.op->ctx->stream;
+  const int groups = std::max(1, 256 / K.k), cw = std::max(1, std::min(K.k, 32 / groups));
   timed_launch(K.op->ctx, KC_KRYLOV, [&] {
-    k_mdot<S><<<1, 256, 0, s>>>(static_cast<const S*>(x), 0, static_cast<const S*>(x), K.N, K.k, K.hdev.as<S>());
+    k_mdot<S><<<(K.k + cw - 1) / cw, groups * cw, 0, s>>>(static_cast<const S*>(x), K.N, K.k, groups, cw,
+                                                         K.hdev.as<S>());
     return cudaGetLastError();
   });
   std::vector<HostS<S>> h(K.k);
@@ -281,24 +307,23 @@ bg_status fgmres(Krylov& K, int prec, Krylov* inner, int inner_prec, double inne
   cudaError_t e = cudaSuccess;
   std::vector<H> Hm((size_t)(m + 1) * m * k), g((size_t)(m + 1) * k), cs((size_t)m * k), sn((size_t)m * k);
   std::vector<H> hcol((size_t)(m + 1) * k);
-  std::vector<double> inv(k), beta;
+  std::vector<double> inv(k), beta = bn;
+  const void* rv = b;  // the residual; x is zero on entry, so the first one is b
   int it = 0;
   bool first_cycle = true;
   while (true) {
-    // true residual r = b - A x (x is zero on entry, so the first one is b)
-    if (first_cycle) {
-      e = cudaMemcpyAsync(r.p, b, nk * sizeof(S), cudaMemcpyDeviceToDevice, s);
-      if (e != cudaSuccess) return cuda_status(op->ctx, e, "gmres");
-      first_cycle = false;
-    } else {
+    // true residual r = b - A x
+    if (!first_cycle) {
       if ((st = apply_operator(op, k, prec, x, r.p, true)) != BG_OK) return st;
       ++(low ? cnt->mixed_mv : cnt->fp64_mv);
       timed_launch(op->ctx, KC_KRYLOV, [&] {
         k_residual<S><<<nblk(nk), 256, 0, s>>>(static_cast<const S*>(b), nk, r.as<S>());
         return cudaGetLastError();
       });
+      rv = r.p;
+      if ((st = col_norms<S>(K, rv, &beta)) != BG_OK) return st;
     }
-    if ((st = col_norms<S>(K, r.p, &beta)) != BG_OK) return st;
+    first_cycle = false;
     bool done = true;
     for (int c = 0; c < k; ++c)
       if (beta[c] > tol * bn[c] && bn[c] > 0) done = false;
@@ -311,7 +336,7 @@ bg_status fgmres(Krylov& K, int prec, Krylov* inner, int inner_prec, double inne
     e = cudaMemcpyAsync(K.inv.p, inv.data(), k * sizeof(double), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return cuda_status(op->ctx, e, "gmres");
     timed_launch(op->ctx, KC_KRYLOV, [&] {
-      k_vscale<S><<<nblk(nk), 256, 0, s>>>(r.as<S>(), K.inv.as<double>(), N, k, K.V.as<S>());
+      k_vscale<S><<<nblk(nk), 256, 0, s>>>(static_cast<const S*>(rv), K.inv.as<double>(), N, k, K.V.as<S>());
       return cudaGetLastError();
     });
     std::fill(Hm.begin(), Hm.end(), H(0));
@@ -351,12 +376,14 @@ bg_status fgmres(Krylov& K, int prec, Krylov* inner, int inner_prec, double inne
         ++(low ? cnt->mixed_mv : cnt->fp64_mv);
         // classical Gram-Schmidt (gs_passes passes: two for the outer and the plain
         // FP64 solve, one for the inner preconditioning solve) and the norm, on the device;
-        // one copy brings the Hessenberg column back
+        // the sums also write the Hessenberg column to its pinned slot
         S* h1 = K.hdev.as<S>();
         S* h2 = h1 + (size_t)(m + 1) * k;
         S* h3 = h2 + (size_t)(m + 1) * k;
+        S* slot = reinterpret_cast<S*>(static_cast<unsigned char*>(K.hpin) + (jj & 1) * K.slot_bytes);
         for (int pass = 0; pass < gs_passes; ++pass) {
           S* hp = pass == 0 ? h1 : h2;
+          S* hs = slot + (size_t)pass * (m + 1) * k;
           // split the rows over enough CTAs to fill the GPU
           const int nch = std::max(1, std::min(64, (4 * 152 + jj) / (jj + 1)));
           const int rows_per = (N + nch - 1) / nch;
@@ -366,7 +393,8 @@ bg_status fgmres(Krylov& K, int prec, Krylov* inner, int inner_prec, double inne
             return cudaGetLastError();
           });
           timed_launch(op->ctx, KC_KRYLOV, [&] {
-            k_reduce_parts<S><<<((jj + 1) * k + 255) / 256, 256, 0, s>>>(K.part.as<S>(), jj + 1, nch, k, hp);
+            k_reduce_parts<S><<<((jj + 1) * k + 255) / 256, 256, 0, s>>>(K.part.as<S>(), jj + 1, nch, k, hp, hs,
+                                                                         nullptr);
             return cudaGetLastError();
           });
           timed_launch(op->ctx, KC_KRYLOV, [&] {
@@ -381,26 +409,16 @@ bg_status fgmres(Krylov& K, int prec, Krylov* inner, int inner_prec, double inne
             return cudaGetLastError();
           });
           timed_launch(op->ctx, KC_KRYLOV, [&] {
-            k_reduce_parts<S><<<(k + 255) / 256, 256, 0, s>>>(K.part.as<S>(), 1, nch, k, h3);
+            k_reduce_parts<S><<<(k + 255) / 256, 256, 0, s>>>(K.part.as<S>(), 1, nch, k, h3,
+                                                             slot + (size_t)2 * (m + 1) * k, K.inv.as<double>());
             return cudaGetLastError();
           });
         }
         timed_launch(op->ctx, KC_KRYLOV, [&] {
-          k_inv_norm<S><<<(k + 63) / 64, 64, 0, s>>>(h3, k, K.inv.as<double>());
-          return cudaGetLastError();
-        });
-        timed_launch(op->ctx, KC_KRYLOV, [&] {
           k_vscale<S><<<nblk(nk), 256, 0, s>>>(K.w.as<S>(), K.inv.as<double>(), N, k, K.V.as<S>() + (long)(jj + 1) * vstride);
           return cudaGetLastError();
         });
-      unsigned char* slot = static_cast<unsigned char*>(K.hpin) + (jj & 1) * K.slot_bytes;
-      e = cudaMemcpyAsync(slot, h1, (size_t)(jj + 1) * k * sizeof(S), cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess && gs_passes > 1)
-        e = cudaMemcpyAsync(slot + (size_t)(m + 1) * k * sizeof(S), h2, (size_t)(jj + 1) * k * sizeof(S),
-                            cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(slot + (size_t)2 * (m + 1) * k * sizeof(S), h3, k * sizeof(S), cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess) e = cudaEventRecord(K.ev[jj & 1], s);
+      e = cudaEventRecord(K.ev[jj & 1], s);
       return cuda_status(op->ctx, e, "gmres orthogonalisation");
     };
     auto process_column = [&](int j, bool* all_done_out) -> bg_status {
