@@ -238,6 +238,106 @@ __global__ void k_potential(const d4* __restrict__ tab, int ne, int Q, const dou
   }
 }
 
+// The same sums for many points and right-hand sides: a lane is a point, a warp
+// an element. The element's moments sum_q k(x, y_q) c_q phi_a(y_q) stay in the
+// lane's registers and meet the coefficients of all columns, so a kernel value
+// is computed once, not once per column, and a column costs (P + 1)^2
+// multiply-adds per element and point instead of Q times the integrand.
+// Bound by the FP64 pipe: 100 points, 32 columns, 6144 elements, P = 2 (Q = 16):
+// 27.1 -> 1.8 ms for the whole call; complex, 16 columns, 1024 elements 5.4 ->
+// 0.77; 32 points, 2 columns 2.0 -> 0.56. A CTA (a chunk of the elements, 32 points) writes its
+// sum to `part`; k_potential_sum adds the chunks' in order.
+constexpr int kPotWarps = 8, kPotCols = 32;  // columns: real values of a batch
+
+template <int P, bool CPLX>
+__global__ void __launch_bounds__(32 * kPotWarps) k_potential_many(
+    const d4* __restrict__ tab, int ne, int Q, int per_chunk, const double* __restrict__ basis,
+    const double* __restrict__ coef, int k, const double* __restrict__ pts, int npts, double kre, double kim,
+    double* __restrict__ part) {
+  constexpr int P2 = (P + 1) * (P + 1), CW = CPLX ? 2 : 1, KB = kPotCols / CW;
+  __shared__ double red[kPotWarps][32][kPotCols / 4 + 1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c0 = blockIdx.z * KB;
+  const int p = min((int)blockIdx.y * 32 + lane, npts - 1);
+  const double px = pts[3 * p], py = pts[3 * p + 1], pz = pts[3 * p + 2];
+  double acc[kPotCols];
+#pragma unroll
+  for (int c = 0; c < kPotCols; ++c) acc[c] = 0;
+  const int e1 = min(ne, (int)(blockIdx.x + 1) * per_chunk);
+  for (int e = blockIdx.x * per_chunk + w; e < e1; e += kPotWarps) {
+    double m[P2][CW];
+#pragma unroll
+    for (int a = 0; a < P2; ++a)
+#pragma unroll
+      for (int v = 0; v < CW; ++v) m[a][v] = 0;
+    for (int q = 0; q < Q; ++q) {
+      const d4 y = tab[(long)e * Q + q];
+      const double d0 = px - y.x, d1 = py - y.y, d2 = pz - y.z;
+      const double r2 = d0 * d0 + d1 * d1 + d2 * d2;
+      const double inv = rsqrt_nr(r2);
+      double kr = inv * kInv4Pi * y.w, ki = 0.0;
+      if (CPLX) {
+        const double r = r2 * inv;
+        double sn, cs;
+        sincos(kre * r, &sn, &cs);
+        const double a = kim != 0.0 ? exp(kim * r) : 1.0;
+        ki = -sn * a * kr;
+        kr = cs * a * kr;
+      }
+#pragma unroll
+      for (int a = 0; a < P2; ++a) {
+        const double b = basis[q * P2 + a];
+        m[a][0] = fma(kr, b, m[a][0]);
+        if (CPLX) m[a][CW - 1] = fma(ki, b, m[a][CW - 1]);
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < P2; ++a) {
+      const double* cf = coef + (((long)e * P2 + a) * k + c0) * CW;
+#pragma unroll
+      for (int c = 0; c < KB; ++c) {
+        if (c0 + c >= k) break;
+        if (CPLX) {
+          const double re = cf[2 * c], im = cf[2 * c + 1];
+          acc[2 * c] = fma(m[a][0], re, fma(-m[a][CW - 1], im, acc[2 * c]));
+          acc[2 * c + CW - 1] = fma(m[a][0], im, fma(m[a][CW - 1], re, acc[2 * c + CW - 1]));
+        } else {
+          acc[c] = fma(m[a][0], cf[c], acc[c]);
+        }
+      }
+    }
+  }
+  // the warps' sums, a quarter of the columns at a time
+  const int kv = k * CW;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < kPotCols / 4; ++c) red[w][lane][c] = acc[h * (kPotCols / 4) + c];
+    __syncthreads();
+    for (int t = threadIdx.x; t < 32 * (kPotCols / 4); t += blockDim.x) {
+      const int l = t / (kPotCols / 4), c = t % (kPotCols / 4);
+      const int pp = blockIdx.y * 32 + l, cc = c0 * CW + h * (kPotCols / 4) + c;
+      if (pp >= npts || cc >= kv) continue;
+      double s = 0;
+#pragma unroll
+      for (int ww = 0; ww < kPotWarps; ++ww) s += red[ww][l][c];
+      part[((long)blockIdx.x * npts + pp) * kv + cc] = s;
+    }
+  }
+}
+
+// out[c][p] (re, im for CW = 2) = sum over the chunks of part[chunk][p][c]
+template <int CW>
+__global__ void k_potential_sum(const double* __restrict__ part, int chunks, int npts, int k,
+                                double* __restrict__ out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, kv = k * CW;
+  if (t >= npts * kv) return;
+  double s = 0;
+  for (int ch = 0; ch < chunks; ++ch) s += part[(long)ch * npts * kv + t];
+  const int p = t / kv, c = t % kv;
+  out[((long)(c / CW) * npts + p) * CW + c % CW] = s;
+}
+
 // Maxwell field (Maxwell/SingleLayerPotential.hpp:44-95 with the div-conforming
 // evaluator of AnsatzSpace/FunctionEvaluatorEval.hpp:39-83): CTA per evaluation
 // point x; threads over (element, Gauss point y) sum, with weight h^2 w,
@@ -353,8 +453,48 @@ cudaError_t launch_load(int G, int P, bool cplx, const PatchTable& pt, const Ele
     default: return cudaErrorInvalidValue;
   }
 }
+// Elements per CTA of k_potential_many: whole warps' turns, so that the CTAs of
+// all points and columns are about four per SM; with many points one chunk holds
+// all elements, so the partial sums stay below 608 x 32 points' or the output's size
+int potential_per_chunk(bool cplx, int ne, int npts, int k) {
+  const long ctas = (long)((npts + 31) / 32) * ((k * (cplx ? 2 : 1) + kPotCols - 1) / kPotCols);
+  const long chunks = std::max(1L, 4 * 152 / std::max(1L, ctas));
+  return (int)((ne + chunks * kPotWarps - 1) / (chunks * kPotWarps)) * kPotWarps;
+}
+// Whether the points and columns fill its warps: a warp works on 32 points, and
+// the integrands that the kernel of one point computes again for each column
+// are what it saves. One column is left to that kernel: 1.13 ms for 8 to 100
+// points (6144 elements, P = 2), where 8 points and 32 columns are 27 -> 0.9.
+bool potential_many(int npts, int k) { return npts >= 8 && k >= 2 && (long)npts * k >= 64 && npts <= (1 << 20); }
+// part: with it, the kernel for many points and columns, ceil(ne / per_chunk) npts k values
 cudaError_t launch_potential(int P, bool cplx, const d4* tab, int ne, int Q, const double* basis, const double* coef,
-                             int k, const double* pts, int npts, double kre, double kim, double* out, cudaStream_t s) {
+                             int k, const double* pts, int npts, double kre, double kim, double* part, int per_chunk,
+                             double* out, cudaStream_t s) {
+  if (part) {
+    const int cw = cplx ? 2 : 1, chunks = (ne + per_chunk - 1) / per_chunk;
+    const dim3 grid(chunks, (npts + 31) / 32, (k * cw + kPotCols - 1) / kPotCols);
+#define BG_POT(PP)                                                                                        \
+  case PP:                                                                                                \
+    if (cplx)                                                                                             \
+      k_potential_many<PP, true><<<grid, 32 * kPotWarps, 0, s>>>(tab, ne, Q, per_chunk, basis, coef, k,   \
+                                                                 pts, npts, kre, kim, part);              \
+    else                                                                                                  \
+      k_potential_many<PP, false><<<grid, 32 * kPotWarps, 0, s>>>(tab, ne, Q, per_chunk, basis, coef, k,  \
+                                                                  pts, npts, kre, kim, part);             \
+    break;
+    switch (P) {
+      BG_POT(0)
+      BG_POT(1)
+      BG_POT(2)
+      BG_POT(3)
+      default: return cudaErrorInvalidValue;
+    }
+#undef BG_POT
+    const int n = npts * k * cw, blocks = (n + 127) / 128;
+    if (cplx) k_potential_sum<2><<<blocks, 128, 0, s>>>(part, chunks, npts, k, out);
+    else k_potential_sum<1><<<blocks, 128, 0, s>>>(part, chunks, npts, k, out);
+    return cudaGetLastError();
+  }
 #define BG_POT(PP)                                                                                              \
   case PP:                                                                                                      \
     if (cplx) k_potential<PP, true><<<npts, 256, 0, s>>>(tab, ne, Q, basis, coef, k, pts, kre, kim, out);      \
@@ -518,7 +658,7 @@ extern "C" bg_status bg_potential(bg_operator* op, const void* rho, int nrhs, co
   }
   PatchTable pt{op->d_patch_meta.as<int>(), op->d_patch_cp.as<double>()};
   ElementTable et{op->d_el_patch.as<int>(), op->d_el_llc.as<double>(), 1.0 / double(1 << op->M)};
-  DevBuf gx, gw, tab, dbas, dpts, drho, dout;
+  DevBuf gx, gw, tab, dbas, dpts, drho, dout, part;
   std::vector<double> P3(pts, pts + 3 * npts);
   cudaError_t e = gx.upload(gr.x, s);
   if (e == cudaSuccess) e = gw.upload(gr.w, s);
@@ -540,9 +680,14 @@ extern "C" bg_status bg_potential(bg_operator* op, const void* rho, int nrhs, co
       e = launch_csr_apply(op->stype(false), op->d_T_ptr.as<int>(), op->d_T_idx.as<int>(), op->d_T_val.as<double>(),
                            op->S, op->w_xdof.p, op->w_xss.p, k, s);
     if (e == cudaSuccess) e = dout.alloc((size_t)npts * k * usz);
+    const bool many = potential_many(npts, k);
+    const int per_chunk = potential_per_chunk(op->cplx, op->ne, npts, k);
+    if (e == cudaSuccess && many)
+      e = part.alloc((size_t)((op->ne + per_chunk - 1) / per_chunk) * npts * k * usz);
     if (e == cudaSuccess)
       e = launch_potential(op->P, op->cplx, tab.as<d4>(), op->ne, Q, dbas.as<double>(), op->w_xss.as<double>(), k,
-                           dpts.as<double>(), npts, op->kre, op->kim, dout.as<double>(), s);
+                           dpts.as<double>(), npts, op->kre, op->kim, many ? part.as<double>() : nullptr, per_chunk,
+                           dout.as<double>(), s);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(static_cast<char*>(out) + (size_t)c0 * npts * usz, dout.p, (size_t)npts * k * usz,
                           cudaMemcpyDeviceToHost, s);

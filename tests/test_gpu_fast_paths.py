@@ -152,3 +152,17 @@ def test_solver_sums_for_any_number_of_columns(ctx, kind, nrhs):
     x, _ = A.solve(b, tol=1e-9, inner="fp64")
     r = np.linalg.norm(A.matvec(x) - b, axis=0) / np.linalg.norm(b, axis=0)
     assert r.max() < 2e-9
+
+
+@pytest.mark.parametrize("kind,P", [(0, 0), (0, 2), (1, 1), (1, 3)])
+@pytest.mark.parametrize("npts,nrhs", [(64, 2), (8, 8), (33, 16), (100, 32), (31, 40), (700, 17)])
+def test_potential_of_many_columns(ctx, kind, P, npts, nrhs):
+    """The potential with lanes as points and all columns at once: the same
+    sums as one column at a time up to their order (1e-13 of the largest)."""
+    d = _operator(ctx, SPHERE, 1, P, kind, 1.3)
+    rng = np.random.default_rng(12)
+    rho = rng.normal(size=(d.N, nrhs)) + (1j * rng.normal(size=(d.N, nrhs)) if kind else 0)
+    pts = rng.uniform(-0.4, 0.4, (npts, 3))
+    y = d.potential(rho, pts)
+    z = np.stack([np.asarray(d.potential(rho[:, c:c + 1], pts)).reshape(npts) for c in range(nrhs)], 1)
+    assert np.abs(np.asarray(y).reshape(npts, nrhs) - z).max() < 1e-13 * np.abs(z).max()
