@@ -26,6 +26,8 @@ static void context_free(bg_context* ctx) {
       }
     for (auto ev : ctx->event_pool) cudaEventDestroy(ev);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    for (auto& ev : ctx->side_ev) cudaEventDestroy(ev);
+    cudaStreamDestroy(ctx->side);
     cudaStreamDestroy(ctx->stream);
   }
   delete ctx;
@@ -84,7 +86,15 @@ bg_status bg_context_create(int device, bg_context** out) {
       delete ctx;
       return BG_DEVICE_ERROR;
     }
-    if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) {
+    bool ok = cudaSetDevice(device) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) == cudaSuccess;
+    for (auto& ev : ctx->side_ev) ok = ok && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess;
+    if (!ok) {
+      for (auto& ev : ctx->side_ev)
+        if (ev) cudaEventDestroy(ev);
+      if (ctx->side) cudaStreamDestroy(ctx->side);
+      if (ctx->stream) cudaStreamDestroy(ctx->stream);
       delete ctx;
       return BG_DEVICE_ERROR;
     }
@@ -1559,7 +1569,9 @@ static bool near_by_digits(const bg_operator* op, const DevBuf& dig, int nc, boo
   return nc > 2 || (nc == 2 && (op->cplx || op->dense.B > 16));
 }
 // columns c0 .. c0 + nc - 1 (rows of ld scalars) of the near field
-static cudaError_t oz_near_product(const bg_operator* op, const DevBuf& dense64, const DevBuf& dig, int ld, int c0, int nc) {
+constexpr int kOzFmax = 2 * kOzMaxSegs * 32;
+static cudaError_t oz_near_product(const bg_operator* op, const DevBuf& dense64, const DevBuf& dig, int ld, int c0, int nc,
+                                   cudaStream_t s) {
   OzArgs a{};
   a.seg[0] = oz_near_seg(op, dense64, dig);
   a.nseg = 1;
@@ -1569,9 +1581,9 @@ static cudaError_t oz_near_product(const bg_operator* op, const DevBuf& dense64,
   a.c0 = c0;
   a.ncols = nc;
   a.pass_panels = (size_t)op->dense.nrows * bsr_oz_panel_bytes(a.B, op->cplx);
-  a.fmax = op->w_oz_fmax.as<int>();
+  a.fmax = op->w_oz_fmax.as<int>() + kOzFmax;  // the far field has the first half and may run beside
   a.err = op->d_err.as<int>();
-  return launch_bsr_oz(op->cplx, false, a, op->near_row_max, op->oz_near_passes, op->ctx->stream);
+  return launch_bsr_oz(op->cplx, false, a, op->near_row_max, op->oz_near_passes, s);
 }
 // the far field of every level with couplings df, y[l] to z[l]
 static cudaError_t oz_far_product(const bg_operator* op, const std::vector<DevBuf*>& df, const std::vector<DevBuf*>& y,
@@ -1641,7 +1653,7 @@ bg_status ensure_work(bg_operator* op, int nrhs) {
     const int cols = op->maxwell() ? 4 * std::min(nrhs, (int)bg_operator::kMwRhsChunk) : nrhs;
     op->oz_far_passes = oz_passes(op, op->n_far_work, cols);
     if (op->far_oz) BG_CHECK(op->w_oz_far.alloc(oz_far_panels(op, nullptr) * op->oz_far_passes), "work vectors");
-    BG_CHECK(op->w_oz_fmax.alloc((size_t)2 * kOzMaxSegs * 32 * sizeof(int)), "work vectors");
+    BG_CHECK(op->w_oz_fmax.alloc((size_t)2 * kOzFmax * sizeof(int)), "work vectors");
   }
   if (op->fmm_fused) {
     // arrival counters of the fused upward pass: parents at levels
@@ -1692,7 +1704,13 @@ static void fill_fmm(const bg_operator* op, const void* fac, int kk, const void*
 // The product between T x and T^T y: superspace x in w_xss to superspace y in
 // w_yss, only on the operator's own work buffers (so it can be captured as a
 // CUDA graph and replayed).
-static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver) {
+// beside (a capture): the near field as a branch of its own from the input on to
+// the backward transforms, which add to its result. Neither path fills the chip
+// by itself: the transforms wait for memory and the FP64 pipe, the near field
+// mostly for shared memory, and small sizes for launches. Whole products, one
+// after the other -> beside: Laplace M = 2, one column, FP64 130 -> 116 us; M = 5,
+// 32 columns, mixed 764 -> 722; Helmholtz M = 3, 16 columns, mixed 738 -> 601.
+static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver, bool beside = false) {
   cudaStream_t s = op->ctx->stream;
   const bool mixed = prec != BG_PREC_FP64;   // far field and transforms in FP32
   const bool near32 = prec == BG_PREC_FP32;  // near field in FP32 too
@@ -1703,6 +1721,14 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver) 
   const bg_launch_plan pl = op->plan_for(nrhs, prec);
   bool any_far = false;
   for (const auto& f : op->far) any_far |= !f.col.empty();
+  beside = beside && any_far && !op->kbatched();
+  const cudaStream_t sn = beside ? op->ctx->side : s;  // the near field's
+  if (near32 && !op->kbatched())
+    BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_convert(S64, Sfar, op->w_xss.p, ss_n, op->w_xss32.p, s); }), "x to FP32");
+  if (beside) {
+    BG_CHECK(cudaEventRecord(op->ctx->side_ev[0], s), "near-field branch");
+    BG_CHECK(cudaStreamWaitEvent(sn, op->ctx->side_ev[0], 0), "near-field branch");
+  }
   if (op->kbatched()) {
     // batched wavenumbers: wavenumber q's near field on column block q (the
     // block is copied out of the row-major superspace vectors and back)
@@ -1715,7 +1741,7 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver) 
     for (int q = 0; q < nk; ++q) {
       const bg_operator::KSlot& k = op->kslots[q];
       if (!near32 && near_by_digits(op, k.dense_dig, nr, solver)) {
-        BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return oz_near_product(op, k.dense64, k.dense_dig, nrhs, q * nr, nr); }),
+        BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return oz_near_product(op, k.dense64, k.dense_dig, nrhs, q * nr, nr, s); }),
                  "near-field product (batched wavenumbers, tensor cores)");
         continue;
       }
@@ -1734,19 +1760,18 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver) 
     }
   } else if (near32) {
     // FP32 near field into the FP32 accumulator the far field adds to
-    BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_convert(S64, Sfar, op->w_xss.p, ss_n, op->w_xss32.p, s); }), "x to FP32");
     BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return launch_bsr_fp32(op->cplx, op->dense.d_row_ptr.as<int>(), op->dense.d_col.as<int>(), op->d_dense32.p,
-                        op->block_stride32(op->dense.B), op->dense.nrows, op->dense.B, op->w_xss32.p, op->w_yss32.p, nrhs, 0, s, pl.near_kernel); }),
+                        op->block_stride32(op->dense.B), op->dense.nrows, op->dense.B, op->w_xss32.p, op->w_yss32.p, nrhs, 0, sn, pl.near_kernel); }),
              "near-field product (FP32)");
   } else if ((!mixed || pl.mixed_near == 0) && near_by_digits(op, op->d_dense_dig, nrhs, solver)) {
     // FP64-accurate near field on the tensor cores: 8 integer digits of 7
     // bits per operand, exact integer accumulation, one rounding at the end
-    BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return oz_near_product(op, op->d_dense64, op->d_dense_dig, nrhs, 0, nrhs); }),
+    BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return oz_near_product(op, op->d_dense64, op->d_dense_dig, nrhs, 0, nrhs, sn); }),
              "near-field product (tensor cores, integer digits)");
   } else if (mixed && !op->cplx && op->d_dense_df.p && (pl.mixed_near != 0 || !op->near_oz)) {
     // FP64-accurate near field in double-float: blocks and x as FP32 (hi, lo)
     // pairs, exact products and compensated sums (about 1e-14 relative)
-    BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_split_df(op->w_xss.p, ss_n, op->w_xss_df.p, s); }),
+    BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_split_df(op->w_xss.p, ss_n, op->w_xss_df.p, sn); }),
              "near-field split of x");
     // launch plan: 32 columns with a quarter of them on the FP64 pipe, the
     // rest in double-float
@@ -1755,16 +1780,17 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver) 
                return both_pipes
                           ? launch_bsr_near_mix(op->dense.d_row_ptr.as<int>(), op->dense.d_col.as<int>(), op->d_dense_df.p,
                                                 op->d_dense64.p, op->block_stride(op->dense.B), op->dense.nrows, op->dense.B,
-                                                op->w_xss_df.p, op->w_xss.p, op->w_yss.p, s)
+                                                op->w_xss_df.p, op->w_xss.p, op->w_yss.p, sn)
                           : launch_bsr_df(op->dense.d_row_ptr.as<int>(), op->dense.d_col.as<int>(), op->d_dense_df.p,
                                           op->block_stride(op->dense.B), op->dense.nrows, op->dense.B, op->w_xss_df.p,
-                                          op->w_yss.p, nrhs, 0, s); }),
+                                          op->w_yss.p, nrhs, 0, sn); }),
              "near-field product (double-float)");
   } else {
     BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return launch_bsr_fp64(op->cplx, op->dense.d_row_ptr.as<int>(), op->dense.d_col.as<int>(), op->d_dense64.p,
-                        op->block_stride(op->dense.B), op->dense.nrows, op->dense.B, op->w_xss.p, op->w_yss.p, nrhs, 0, s); }),
+                        op->block_stride(op->dense.B), op->dense.nrows, op->dense.B, op->w_xss.p, op->w_yss.p, nrhs, 0, sn); }),
              "near-field product");
   }
+  if (beside) BG_CHECK(cudaEventRecord(op->ctx->side_ev[1], sn), "near-field branch");
   if (any_far) {
     const long comp_ss = (long)op->ne * op->p2;  // superspace rows per vector component
     const void* xfar = op->w_xss.p;
@@ -2076,6 +2102,7 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver) 
                    "far-field product");
       }
     }
+    if (beside) BG_CHECK(cudaStreamWaitEvent(s, op->ctx->side_ev[1], 0), "near-field branch");
     if (op->maxwell()) {
       for (int l = 0; l < Ll; ++l) {
         const int nb = 3 * op->nclusters(l);
@@ -2215,7 +2242,7 @@ bg_status apply_operator(bg_operator* op, int nrhs, int prec, const void* xdof, 
       long c0[8];
       for (int c = 0; c < 8; ++c) c0[c] = ctx->class_launches[c];
       cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-      bg_status mst = e == cudaSuccess ? apply_middle(op, nrhs, prec, solver) : BG_DEVICE_ERROR;
+      bg_status mst = e == cudaSuccess ? apply_middle(op, nrhs, prec, solver, true) : BG_DEVICE_ERROR;
       cudaGraph_t g = nullptr;
       if (e == cudaSuccess) e = cudaStreamEndCapture(s, &g);
       bg_operator::ProductGraph pg;

@@ -64,6 +64,8 @@ struct bg_context {
   int children = 0;      // live geometries and operators
   bool closing = false;  // bg_context_destroy was called; free with the last child
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;  // the near field's branch of a captured product
+  cudaEvent_t side_ev[2] = {nullptr, nullptr};
   std::string err;
   DevBuf stage_in, stage_out;   // device staging of host operands
   void* pinned = nullptr;       // pinned host staging

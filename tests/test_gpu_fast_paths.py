@@ -166,3 +166,19 @@ def test_potential_of_many_columns(ctx, kind, P, npts, nrhs):
     y = d.potential(rho, pts)
     z = np.stack([np.asarray(d.potential(rho[:, c:c + 1], pts)).reshape(npts) for c in range(nrhs)], 1)
     assert np.abs(np.asarray(y).reshape(npts, nrhs) - z).max() < 1e-13 * np.abs(z).max()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp32"])
+@pytest.mark.parametrize("kind,nrhs", [(0, 1), (0, 33), (1, 1), (1, 5), (2, 3)])
+def test_near_field_beside_the_far_field(ctx, kind, nrhs, precision):
+    """From the second product of a shape on, the near field is a branch of a
+    graph beside the transforms and the far field: the same bits as the first
+    product's launches in a row, also after another shape in between."""
+    d = _operator(ctx, SPHERE, 3, 1, kind, 1.1)
+    A = d.get_discrete_operator()
+    rng = np.random.default_rng(13)
+    x = rng.normal(size=(d.N, nrhs)) + (1j * rng.normal(size=(d.N, nrhs)) if kind else 0)
+    y = A.matvec(x, precision=precision)
+    for _ in range(3):
+        assert np.array_equal(A.matvec(x, precision=precision), y)
+        A.matvec(x[:, :1], precision="fp64")
