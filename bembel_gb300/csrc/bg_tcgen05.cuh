@@ -1,8 +1,8 @@
 // Inline-PTX helpers for the 5th-generation tensor cores (tcgen05, sm_103a):
 // shared-memory matrix descriptors, instruction descriptors, MMA issue and
 // commit, bounded mbarrier waits, 1-D TMA bulk copies and tensor-memory
-// loads. Shared by the far-field (bg_far_tc.cu) and near-field
-// (bg_near_tc.cu) tensor-core kernels.
+// loads. Shared by the far-field (bg_far_tc.cu) and the FP64-accurate
+// (bg_bsr_oz.cu) tensor-core kernels.
 #pragma once
 #include <cstdint>
 
