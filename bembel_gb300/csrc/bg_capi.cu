@@ -1869,6 +1869,20 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver, 
                  "forward transfer");
       }
     }
+    // Maxwell: levels l0 .. l1 around the scalar far product, into it (Y to its
+    // columns) or out of it
+    auto mw_levels = [&](bool in, int l0, int l1) {
+      MwFarLevels L{};
+      L.n = std::min(l1 - l0 + 1, kMwFarLevels);
+      for (int i = 0; i < L.n; ++i) {
+        const int l = l0 + i;
+        L.ncl[i] = op->nclusters(l);
+        L.in[i] = in ? op->w_y[l]->p : op->w_zv[l]->p;
+        L.out[i] = in ? op->w_yv[l]->p : op->w_z[l]->p;
+        L.tan[i] = mixed ? op->d_tan32[l]->p : op->d_tan64[l]->p;
+      }
+      return L;
+    };
     const bool tc = mixed && op->vd == 1 && op->nc == 1 && op->leaf_level < kMaxFarLevels &&
                     far_tc_supported(op->cplx, np2, nrhs);
     const bool tcc = mixed && op->cplx && op->far_tiles && op->leaf_level < kMaxFarLevels;
@@ -1954,17 +1968,13 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver, 
         const std::complex<double> kap(op->kre, op->kim), mk2 = -1.0 / (kap * kap);
         for (int r0 = 0; r0 < nrhs; r0 += bg_operator::kMwRhsChunk) {
           const int nr = std::min((int)bg_operator::kMwRhsChunk, nrhs - r0);
-          for (int l = 0; l <= op->leaf_level; ++l)
-            BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_in(Sfar, op->nclusters(l), np2, op->w_y[l]->p, nrhs,
-                                                                            r0, nr, op->d_tan32[l]->p, op->w_yv[l]->p, s); }),
-                     "Maxwell far-field columns");
+          BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_in(Sfar, mw_levels(true, 0, op->leaf_level), np2, nrhs, r0, nr, s); }),
+                   "Maxwell far-field columns");
           for (int c0 = 0; c0 < 4 * nr; c0 += 16)
             if ((st = product(4 * nr, c0, std::min(16, 4 * nr - c0))) != BG_OK) return st;
-          for (int l = 0; l <= op->leaf_level; ++l)
-            BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_out(Sfar, op->nclusters(l), np2, op->w_zv[l]->p, nrhs,
-                                                                             r0, nr, op->d_tan32[l]->p, mk2.real(),
-                                                                             mk2.imag(), op->w_z[l]->p, s); }),
-                     "Maxwell far-field columns");
+          BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_out(Sfar, mw_levels(false, 0, op->leaf_level), np2, nrhs, r0, nr,
+                                                                           mk2.real(), mk2.imag(), s); }),
+                   "Maxwell far-field columns");
         }
       }
     } else if (tc) {
@@ -2012,17 +2022,13 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver, 
       const std::complex<double> kap(op->kre, op->kim), mk2 = -1.0 / (kap * kap);
       for (int r0 = 0; r0 < nrhs; r0 += bg_operator::kMwRhsChunk) {
         const int nr = std::min((int)bg_operator::kMwRhsChunk, nrhs - r0);
-        for (int l = 0; l <= op->leaf_level; ++l)
-          BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_in(Sfar, op->nclusters(l), np2, op->w_y[l]->p, nrhs, r0,
-                                                                          nr, op->d_tan64[l]->p, op->w_yv[l]->p, s); }),
-                   "Maxwell far-field columns");
+        BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_in(Sfar, mw_levels(true, 0, op->leaf_level), np2, nrhs, r0, nr, s); }),
+                 "Maxwell far-field columns");
         BG_CHECK(timed_launch(op->ctx, KC_FAR64, [&] { return oz_far_product(op, op->d_far_df, op->w_yv, op->w_zv, 4 * nr, 0, 4 * nr); }),
                  "far-field product (tensor cores, integer digits)");
-        for (int l = 0; l <= op->leaf_level; ++l)
-          BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_out(Sfar, op->nclusters(l), np2, op->w_zv[l]->p, nrhs, r0,
-                                                                           nr, op->d_tan64[l]->p, mk2.real(), mk2.imag(),
-                                                                           op->w_z[l]->p, s); }),
-                   "Maxwell far-field columns");
+        BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_out(Sfar, mw_levels(false, 0, op->leaf_level), np2, nrhs, r0, nr,
+                                                                         mk2.real(), mk2.imag(), s); }),
+                 "Maxwell far-field columns");
       }
     } else if (oz_far) {
       // batched wavenumbers: wavenumber q's couplings on column block q
@@ -2045,12 +2051,10 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver, 
         if (!mixed && !op->store_far)
           return set_error(op->ctx, BG_UNSUPPORTED, "the FP64 product needs the stored far field");
         const int ncl = op->nclusters(l);
-        const void* tan = mixed ? (const void*)op->d_tan32[l]->p : (const void*)op->d_tan64[l]->p;
         const std::complex<double> kap(op->kre, op->kim), mk2 = -1.0 / (kap * kap);
         for (int r0 = 0; r0 < nrhs; r0 += bg_operator::kMwRhsChunk) {
           const int nr = std::min((int)bg_operator::kMwRhsChunk, nrhs - r0);
-          BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_in(Sfar, ncl, np2, op->w_y[l]->p, nrhs, r0, nr,
-                                                                          tan, op->w_yv[l]->p, s); }),
+          BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_in(Sfar, mw_levels(true, l, l), np2, nrhs, r0, nr, s); }),
                    "Maxwell far-field columns");
           if (mixed)
             BG_CHECK(timed_launch(op->ctx, KC_FAR_FUSED, [&] { return launch_far_fused(true, op->d_pts32[l]->as<float4>(), op->d_centres[l]->as<d4>(),
@@ -2064,8 +2068,8 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver, 
             BG_CHECK(timed_launch(op->ctx, KC_FAR64, [&] { return launch_bsr_fp64(true, f.d_row_ptr.as<int>(), f.d_col.as<int>(), op->d_far64[l]->p,
                                   op->block_stride(f.B), f.nrows, f.B, op->w_yv[l]->p, op->w_zv[l]->p, 4 * nr, 0, s); }),
                      "far-field product (Maxwell)");
-          BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_out(Sfar, ncl, np2, op->w_zv[l]->p, nrhs, r0, nr, tan,
-                                                                           mk2.real(), mk2.imag(), op->w_z[l]->p, s); }),
+          BG_CHECK(timed_launch(op->ctx, KC_OTHER, [&] { return launch_mw_far_out(Sfar, mw_levels(false, l, l), np2, nrhs, r0, nr,
+                                                                           mk2.real(), mk2.imag(), s); }),
                    "Maxwell far-field columns");
         }
         continue;

@@ -2,6 +2,8 @@
 // (interpolationPoints2D / map2surface, H2Multipole.hpp:324-375) and the FP64
 // coupling blocks F_ij = k(x_i, y_j) |J(x_i)| |J(y_j)| of the low-rank leaves
 // (Laplace/Helmholtz SingleLayerOperator::evaluateFMMInterpolation_impl, :87-110).
+#include <algorithm>
+
 #include "bg_kernels.cuh"
 
 namespace bg {
@@ -111,11 +113,16 @@ cudaError_t launch_far_assemble(bool cplx, const d4* pts, const int2* pairs, int
 
 // ---------------------------------------------------------------------------
 // Maxwell far field around the scalar kernel product. One thread per
-// (cluster, point, right-hand side of the chunk); the three channels of Y and
-// Z are [channel][cluster][np2][nrhs].
+// (cluster, point, right-hand side of the chunk), blockIdx.y the level: a level
+// by itself is a launch of a few microseconds, mostly latency (all levels in
+// one: a solve of sphere M = 3, 8 columns, 574 products, 217 -> 212 ms).
+// The three channels of Y and Z are [channel][cluster][np2][nrhs].
 template <typename S, typename R>
-__global__ void k_mw_far_in(int ncl, int np2, const S* __restrict__ y, int nrhs, int r0, int nr,
-                            const R* __restrict__ tan, S* __restrict__ yv) {
+__global__ void k_mw_far_in(const __grid_constant__ MwFarLevels L, int np2, int nrhs, int r0, int nr) {
+  const int ncl = L.ncl[blockIdx.y];
+  const S* __restrict__ y = static_cast<const S*>(L.in[blockIdx.y]);
+  const R* __restrict__ tan = static_cast<const R*>(L.tan[blockIdx.y]);
+  S* __restrict__ yv = static_cast<S*>(L.out[blockIdx.y]);
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long)ncl * np2 * nr) return;
   const int r = (int)(idx % nr);
@@ -131,8 +138,11 @@ __global__ void k_mw_far_in(int ncl, int np2, const S* __restrict__ y, int nrhs,
 }
 
 template <typename S, typename R>
-__global__ void k_mw_far_out(int ncl, int np2, const S* __restrict__ zv, int nrhs, int r0, int nr,
-                             const R* __restrict__ tan, S m, S* __restrict__ z) {
+__global__ void k_mw_far_out(const __grid_constant__ MwFarLevels L, int np2, int nrhs, int r0, int nr, S m) {
+  const int ncl = L.ncl[blockIdx.y];
+  const S* __restrict__ zv = static_cast<const S*>(L.in[blockIdx.y]);
+  const R* __restrict__ tan = static_cast<const R*>(L.tan[blockIdx.y]);
+  S* __restrict__ z = static_cast<S*>(L.out[blockIdx.y]);
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long)ncl * np2 * nr) return;
   const int r = (int)(idx % nr);
@@ -147,33 +157,27 @@ __global__ void k_mw_far_out(int ncl, int np2, const S* __restrict__ zv, int nrh
   z[2 * ch + row] = v[3 * nr] * m;
 }
 
-cudaError_t launch_mw_far_in(int S, int ncl, int np2, const void* y, int nrhs, int r0, int nr, const void* tan,
-                             void* yv, cudaStream_t s) {
-  const long n = (long)ncl * np2 * nr;
-  if (n == 0) return cudaSuccess;
-  const unsigned grid = (unsigned)((n + 255) / 256);
-  if (S == 1)
-    k_mw_far_in<cd, double><<<grid, 256, 0, s>>>(ncl, np2, (const cd*)y, nrhs, r0, nr, (const double*)tan, (cd*)yv);
-  else if (S == 3)
-    k_mw_far_in<cf, float><<<grid, 256, 0, s>>>(ncl, np2, (const cf*)y, nrhs, r0, nr, (const float*)tan, (cf*)yv);
-  else
-    return cudaErrorInvalidValue;
+static dim3 mw_far_grid(const MwFarLevels& L, int np2, int nr) {
+  int most = 0;
+  for (int l = 0; l < L.n; ++l) most = std::max(most, L.ncl[l]);
+  return dim3((unsigned)(((long)most * np2 * nr + 255) / 256), L.n);
+}
+cudaError_t launch_mw_far_in(int S, const MwFarLevels& L, int np2, int nrhs, int r0, int nr, cudaStream_t s) {
+  const dim3 grid = mw_far_grid(L, np2, nr);
+  if (grid.x == 0 || grid.y == 0) return cudaSuccess;
+  if (S == 1) k_mw_far_in<cd, double><<<grid, 256, 0, s>>>(L, np2, nrhs, r0, nr);
+  else if (S == 3) k_mw_far_in<cf, float><<<grid, 256, 0, s>>>(L, np2, nrhs, r0, nr);
+  else return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
 
-cudaError_t launch_mw_far_out(int S, int ncl, int np2, const void* zv, int nrhs, int r0, int nr, const void* tan,
-                              double mre, double mim, void* z, cudaStream_t s) {
-  const long n = (long)ncl * np2 * nr;
-  if (n == 0) return cudaSuccess;
-  const unsigned grid = (unsigned)((n + 255) / 256);
-  if (S == 1)
-    k_mw_far_out<cd, double><<<grid, 256, 0, s>>>(ncl, np2, (const cd*)zv, nrhs, r0, nr, (const double*)tan,
-                                                  cd{mre, mim}, (cd*)z);
-  else if (S == 3)
-    k_mw_far_out<cf, float><<<grid, 256, 0, s>>>(ncl, np2, (const cf*)zv, nrhs, r0, nr, (const float*)tan,
-                                                 cf{(float)mre, (float)mim}, (cf*)z);
-  else
-    return cudaErrorInvalidValue;
+cudaError_t launch_mw_far_out(int S, const MwFarLevels& L, int np2, int nrhs, int r0, int nr, double mre, double mim,
+                              cudaStream_t s) {
+  const dim3 grid = mw_far_grid(L, np2, nr);
+  if (grid.x == 0 || grid.y == 0) return cudaSuccess;
+  if (S == 1) k_mw_far_out<cd, double><<<grid, 256, 0, s>>>(L, np2, nrhs, r0, nr, cd{mre, mim});
+  else if (S == 3) k_mw_far_out<cf, float><<<grid, 256, 0, s>>>(L, np2, nrhs, r0, nr, cf{(float)mre, (float)mim});
+  else return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
 

@@ -104,10 +104,15 @@ cudaError_t launch_cluster_points(int G, const PatchTable& pt, int level, int nc
 // (q < 3) and v_3 = Ydiv into Yv ([cluster][np2][4 nr]); mw_far_out maps
 // Zv = K Yv back to the channels of Z: Zphi_rc = sum_q t_rc,q(x_i) Zv_q and
 // Zdiv = m Zv_3 (shared by both row components).
-cudaError_t launch_mw_far_in(int S, int ncl, int np2, const void* y, int nrhs, int r0, int nr, const void* tan,
-                             void* yv, cudaStream_t s);
-cudaError_t launch_mw_far_out(int S, int ncl, int np2, const void* zv, int nrhs, int r0, int nr, const void* tan,
-                              double mre, double mim, void* z, cudaStream_t s);
+constexpr int kMwFarLevels = 32;  // levels of one launch: every depth a cluster tree can have
+struct MwFarLevels {
+  int n, ncl[kMwFarLevels];
+  const void *in[kMwFarLevels], *tan[kMwFarLevels];
+  void* out[kMwFarLevels];
+};
+cudaError_t launch_mw_far_in(int S, const MwFarLevels& L, int np2, int nrhs, int r0, int nr, cudaStream_t s);
+cudaError_t launch_mw_far_out(int S, const MwFarLevels& L, int np2, int nrhs, int r0, int nr, double mre, double mim,
+                              cudaStream_t s);
 // F blocks (B x B, column-major) for the listed cluster pairs of one level
 // block k written at out + k * bstride scalars
 cudaError_t launch_far_assemble(bool cplx, const d4* pts, const int2* pairs, int nblocks, int B, long bstride,
