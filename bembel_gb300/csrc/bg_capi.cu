@@ -1839,12 +1839,14 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver, 
       }
     }
     // scalar operators: one fused launch per direction through the
-    // tensor-product factors, unless the plan asks for the batched GEMMs
+    // tensor-product factors, unless the plan asks for the batched GEMMs or
+    // the panels of so many columns are too large (leaf clusters of 16 or 64
+    // elements, n_p 12 with P = 3)
+    const int kk = (op->cplx ? 2 : 1) * nrhs;
     const bool fused_tr = !op->maxwell() && op->fmm_fused && pl.transforms == 0 &&
-                          ((op->cplx ? 2 : 1) * nrhs + 31) / 32 <= op->fmm_cnt_chunks;
+                          (kk + 31) / 32 <= op->fmm_cnt_chunks && fmm_fits(Sfar, op->np, op->fmm_w1, kk);
     FmmLevelsAny fa{};
     if (fused_tr) {
-      const int kk = (op->cplx ? 2 : 1) * nrhs;
       if (mixed) fill_fmm<float>(op, op->d_fmm_fac32.p, kk, xc0, yfar, &fa.f32);
       else fill_fmm<double>(op, op->d_fmm_fac64.p, kk, xc0, yfar, &fa.f64);
       BG_CHECK(timed_launch(op->ctx, KC_TRANSFORM, [&] { return launch_fmm_up(Sfar, fa, op->fmm_hfac.data(), op->nclusters(Ll - 1), s); }),

@@ -659,27 +659,45 @@ size_t fmm_smem_bytes(int np, int w1, int Bq, int nc, bool with_x) {
          sizeof(int) * (size_t)w1 * w1;
 }
 
+// shared memory of the run-time-size passes: the device's 227 KB a CTA, less a
+// kilobyte for what the kernels declare themselves
+constexpr size_t kFmmSmem = 226 * 1024;
+
+// Columns of a panel. FP64 products of up to 16 columns: panels as wide as the
+// columns there are, a thread per output row and column (the same sums in the
+// same order). Both passes, 32-column panels of the compiled sizes -> this: P =
+// 2, M = 4 (n_p 9) 338 -> 73 us for one column, 338 -> 198 for 16; M = 5 890
+// -> 91 and 452; M = 3, P = 1 (n_p 6) 94 -> 43 and 75. From 17 columns the
+// panels are full and the compiled sizes are the faster. FP32 has 64 lanes a
+// clock for the same work and is bound by latency, not by the pipe: 32-column
+// panels for any number of columns.
+template <typename T>
+int fmm_cols(int kk) {
+  int nc = kFmmCols;
+  if (sizeof(T) == 8)
+    while (nc > 1 && nc / 2 >= kk) nc /= 2;
+  return nc;
+}
+bool fmm_compiled(int np, int w1) { return np >= 6 && np <= 10 && (w1 == 4 || w1 == 6); }
+
+template <typename T>
+bool fmm_fits_t(int np, int w1, int kk) {
+  const int nc = fmm_cols<T>(kk);
+  if (nc == kFmmCols && fmm_compiled(np, w1)) return true;
+  return fmm_smem_bytes<T>(np, w1, w1 * w1, nc, true) <= kFmmSmem;  // the upward pass needs more
+}
+
 template <typename T>
 cudaError_t fmm_launch(bool up, FmmLevels<T> a, const double* hfac, int nparents, cudaStream_t s) {
   if (nparents == 0 || a.kk == 0) return cudaSuccess;
   if (a.L < 1 || a.L >= kMaxFarLevels || a.np < 2 || a.np > kFmmMaxNp || a.w1 < 1 || a.w1 * a.w1 != a.Bq ||
-      a.w1 > 16)
+      a.w1 > 16 || !hfac)
     return cudaErrorInvalidValue;
-  // FP64 products of up to 16 columns: panels as wide as the columns there
-  // are, a thread per output row and column (the same sums in the same order).
-  // Both passes, 32-column panels of the compiled sizes -> this: P = 2, M = 4
-  // (n_p 9) 338 -> 73 us for one column, 338 -> 198 for 16; M = 5 890
-  // -> 91 and 452; M = 3, P = 1 (n_p 6) 94 -> 43 and 75. From 17 columns the
-  // panels are full and the compiled sizes are the faster. FP32 has 64 lanes a
-  // clock for the same work and is bound by latency, not by the pipe: 32-column
-  // panels for any number of columns.
-  a.nc = kFmmCols;
-  if (sizeof(T) == 8)
-    while (a.nc > 1 && a.nc / 2 >= a.kk) a.nc /= 2;
+  a.nc = fmm_cols<T>(a.kk);
   // compiled sizes: n_p 6 .. 10 with P = 1, 2 (w1 = 4, 6). Both passes at run
   // time sizes -> compiled, 32 columns: n_p 8, M = 5, P = 1, FP32 229 -> 53 us,
   // FP64 612 -> 581; n_p 7, complex, M = 2, P = 1, FP32 75 -> 20, FP64 115 -> 92
-  if (hfac && a.nc == kFmmCols) {
+  if (a.nc == kFmmCols && fmm_compiled(a.np, a.w1)) {
 #define BG_FMM_T(NPV, W1V) \
   if (a.np == NPV && a.w1 == W1V) return fmm_launch_t<T, NPV, W1V>(up, a, hfac, nparents, s);
     BG_FMM_T(6, 4) BG_FMM_T(6, 6) BG_FMM_T(7, 4) BG_FMM_T(7, 6) BG_FMM_T(8, 4)
@@ -687,7 +705,7 @@ cudaError_t fmm_launch(bool up, FmmLevels<T> a, const double* hfac, int nparents
 #undef BG_FMM_T
   }
   const size_t smem = fmm_smem_bytes<T>(a.np, a.w1, a.Bq, a.nc, up);
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  if (smem > kFmmSmem) return cudaErrorInvalidValue;  // callers ask fmm_fits first
   auto kf = up ? k_fmm_up<T> : k_fmm_down<T>;
   cudaError_t e = smem_limit(kf, smem);
   if (e != cudaSuccess) return e;
@@ -700,6 +718,9 @@ cudaError_t fmm_launch(bool up, FmmLevels<T> a, const double* hfac, int nparents
 
 }  // namespace
 
+bool fmm_fits(int S, int np, int w1, int kk) {
+  return S < 2 ? fmm_fits_t<double>(np, w1, kk) : fmm_fits_t<float>(np, w1, kk);
+}
 cudaError_t launch_fmm_up(int S, const FmmLevelsAny& a, const double* hfac, int nparents, cudaStream_t s) {
   if (S < 2) return fmm_launch<double>(true, a.f64, hfac, nparents, s);
   return fmm_launch<float>(true, a.f32, hfac, nparents, s);

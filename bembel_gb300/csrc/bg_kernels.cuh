@@ -310,7 +310,10 @@ struct FmmLevelsAny {
 // downward pass (transposed transfers, transposed moments added to out);
 // nparents = clusters of level L - 1; S the bg vector type of the pass;
 // hfac the factors on the host (FP64, layout of fac) for the compiled sizes,
-// whose kernels take them as launch parameters (nullptr: generic kernels)
+// whose kernels take them as launch parameters. fmm_fits: whether passes of kk
+// real columns have the shared memory they need; without it the launches
+// return cudaErrorInvalidValue
+bool fmm_fits(int S, int np, int w1, int kk);
 cudaError_t launch_fmm_up(int S, const FmmLevelsAny& a, const double* hfac, int nparents, cudaStream_t s);
 cudaError_t launch_fmm_down(int S, const FmmLevelsAny& a, const double* hfac, int nparents, cudaStream_t s);
 // op(A) of an FMM transform, stored transposed: AT[q][i], q < Ki, i < ld

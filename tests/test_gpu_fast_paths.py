@@ -182,3 +182,27 @@ def test_near_field_beside_the_far_field(ctx, kind, nrhs, precision):
     for _ in range(3):
         assert np.array_equal(A.matvec(x, precision=precision), y)
         A.matvec(x[:, :1], precision="fp64")
+
+
+@pytest.mark.parametrize("P,np_,mcl", [(2, 6, 2), (2, 9, 2), (3, 11, 2), (1, 11, 3), (3, 12, 1)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_transforms_of_large_panels(ctx, oracle, P, np_, mcl, kind):
+    """Leaf clusters of 16 and 64 elements and the largest interpolation
+    degree, whose transform panels pass the shared memory of a block at some
+    number of columns, are served at every number of columns and precision
+    (FP64 and the FP64-accurate near field against the oracle to 1e-12; the
+    FP32 far field and near field to 1e-4, their rounding of 6e-8 times the
+    condition of the interpolation). n_p = 12 has no FP32 far field at any
+    size, so FP64 only there."""
+    M = 3 if mcl < 3 else 4
+    d = _operator(ctx, SPHERE, M, P, kind, 1.2, np_, min_cluster_level=mcl)
+    assert d.n_lowrank > 0
+    o = oracle.Problem(SPHERE, M, P, kind, kappa=1.2 if kind else 0.0, np_=np_, mcl=mcl)
+    rng = np.random.default_rng(14)
+    x = rng.normal(size=(d.N, 33)) + (1j * rng.normal(size=(d.N, 33)) if kind else 0)
+    ref = o.matvec(x)
+    A = d.get_discrete_operator()
+    for n in (1, 8, 9, 16, 17, 33):
+        for prec, tol in (("fp64", FP64_TOL), ("mixed", 1e-4), ("fp32", 1e-4))[:1 if np_ == 12 else 3]:
+            y = A.matvec(x[:, :n], precision=prec)
+            assert np.linalg.norm(y - ref[:, :n]) < tol * np.linalg.norm(ref[:, :n]), (n, prec)
