@@ -18,10 +18,30 @@
 //  - acc_d = sum_j sum_{s + t = d} a_s x_t for d = 0 .. 7 in FP32 tensor
 //    memory. A product is at most 2^12 and a diagonal holds at most 8 per j,
 //    so over 512 source rows acc_d is an exact integer below 2^24, whatever
-//    the order and rounding of the tensor cores' accumulation; the dropped
-//    d >= 8 terms are below 2^-53 of max |A_i| max |x_c| per term;
+//    the order and rounding of the tensor cores' accumulation;
 //  - the epilogue adds the diagonals into one 64-bit fixed-point sum per
 //    output entry and converts it once to FP64.
+// The error is absolute in 2^(e_i + f_c), which is 4 to 16 times max |A_i| max
+// |x_c|: per term below 2^-55.2 for the dropped digits (seven products of 2^12
+// at 2^-70) and 2^-57 for the rounding of A and x (FP32 pairs: 2^-54.8); these
+// are of either sign, about 2^-57.8 each, and grow with the root of the n
+// terms. A plain FP64 sum errs by up to n 2^-53 of S = sum_j |A_ij| |x_jc|
+// instead. The digits lose to it where S is small against 2^(e_i + f_c): an x of
+// very different sizes, a kernel that decays within the row.
+// Near field: the epilogue bounds S from below by the norms of x over 8 rows
+// and the floors of A over 8 columns, and marks the columns of a block row
+// where four times the digits' error could pass the plain sum's bound; the CTA
+// sums those in FP64 at its end (plain_columns). Columns of normal or smooth
+// values have S some 50 times above the line (B = 4 .. 64). All columns marked
+// cost what the FP64 pipe did: sphere M = 5, P = 2, 32 columns 1.76 ms (1.49 on
+// the pipe, 0.23 unmarked), torus M = 3, 16 complex ones 2.03 (2.59, 0.30).
+// Far field: no row is marked. What an entry loses there is relative to the
+// row's largest coupling times the column's largest x; that x reaches the entry
+// too, through a block of this or another level or the near field, and with a
+// coupling of similar size as long as kernel and surface measure vary little.
+// So the loss stays below n 2^-48 of |A| |x|, the bound of the double-float sums
+// that the digits replace; couplings that spread further within a row keep
+// those sums (kFarSpread in bg_capi.cu).
 //
 // MMA (tcgen05.mma kind::f16, cta_group::1, M = 128, K = 16): the rows of the
 // couplings are the M rows (rows beyond B produce accumulator lanes nobody
@@ -33,7 +53,8 @@
 // [Re | Im] of 16 right-hand sides.
 //
 // Roles of a CTA (persistent, one per SM, walking a list of block rows):
-//  warps 0-7   epilogue: tensor-memory quadrant w % 4, half of the columns
+//  warps 0-7   epilogue: tensor-memory quadrant w % 4, half of the columns; warps
+//              0 and 4 also mark the columns that are summed in FP64
 //  warp 8      TMA (1-D bulk copies): the couplings of a stage into the raw
 //              ring, the x digit panels into the stage
 //  warp 9      MMA issue
@@ -48,6 +69,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 #include <cstdint>
 
@@ -73,6 +95,7 @@ constexpr uint32_t kTmemCols = 512;  // two accumulator buffers of 8 diagonals x
 enum { kDigits = 0, kPairsC = 1, kF64C = 2 };
 constexpr int kMaxStages = 4, kMaxRaws = 8;
 constexpr uint32_t kOzSmem = 224 * 1024;
+constexpr uint32_t kPlainSmem = kOzThreads * 8 * sizeof(double);  // partial sums of plain_columns
 
 // the stage geometry of block size B (rows and columns of a block)
 struct OzGeom {
@@ -84,9 +107,13 @@ struct OzGeom {
   uint32_t x_bytes, stage, raw, raw_off;
   int stages, raws;
   uint32_t smem;
-  uint32_t panel;      // bytes of a cluster's digit panels
+  uint32_t panel;      // bytes of a cluster's digit panels and norms
   int chunk_blocks;    // blocks whose diagonals stay exact
 };
+
+// bytes of a cluster's digits, ahead of the norms of its rows: [2 nks][nc] FP32,
+// sum of |x_jc| 2^-f_c over 8 rows (complex: of the real and of the imaginary parts)
+__host__ __device__ constexpr uint32_t oz_norms_at(int nc, int nks) { return 8u * nc * nks * 32u; }
 
 // esz: bytes of a stored entry of a raw slice (FP64 complex: both parts, 16)
 bool oz_geom(int B, bool cplx, int ncols, int esz, OzGeom* g) {
@@ -96,7 +123,7 @@ bool oz_geom(int B, bool cplx, int ncols, int esz, OzGeom* g) {
   g->rg = (B + 7) / 8;
   g->nks = (B + 15) / 16;
   g->nc = cplx || ncols > 16 ? 32 : 16;
-  g->panel = 8u * g->nc * g->nks * 32u;
+  g->panel = oz_norms_at(g->nc, g->nks) + (uint32_t)g->nc * g->nks * 2u * sizeof(float);
   g->chunk_blocks = std::max(1, 512 / (B * (cplx ? 2 : 1)));
   // a stage holds up to three K steps, as many as the converters take in one
   // go: 2 kw groups of 8 columns for each of the B rows
@@ -119,7 +146,7 @@ bool oz_geom(int B, bool cplx, int ncols, int esz, OzGeom* g) {
   const uint32_t over = (uint32_t)(16 - g->rg) * steps * 256u;
   auto need = [&]() {
     const uint32_t after = g->x_bytes + g->raws * g->raw;
-    return g->stages * g->stage + g->raws * g->raw + (over > after ? over - after : 0u);
+    return std::max(kPlainSmem, g->stages * g->stage + g->raws * g->raw + (over > after ? over - after : 0u));
   };
   for (g->stages = kMaxStages; g->stages >= 2; --g->stages)
     for (g->raws = kMaxRaws; g->raws >= 3; --g->raws)
@@ -394,65 +421,186 @@ __device__ __forceinline__ void tmem_ld2(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr));
 }
 
-// Output entry (row i of item, column c) of a column that holds Inf or NaN:
-// plain FP64 sums, so that such values travel as in any FP64 product
+// |v| 2^-e in FP32, rounded down, for |v| < 2^(e + 128); what is below the range
+// of FP32 counts as its smallest number
+__device__ __forceinline__ float scaled_magnitude(double v, int e) {
+  const uint32_t h = (uint32_t)__double2hiint(v) & 0x7FFFFFFFu, l = (uint32_t)__double2loint(v);
+  const int ex = (int)(h >> 20) - e - 896;
+  if ((h | l) == 0u) return 0.0f;
+  return ex <= 0 || h < 0x100000u ? FLT_MIN : __uint_as_float((uint32_t)ex << 23 | (h & 0xFFFFFu) << 3 | l >> 29);
+}
+
+// The columns (bits 0 .. 15) of half h of a pass (complex: of the pass) that have
+// to be summed in FP64 in block row `row`: those with Inf or NaN, and those
+// where the bound of S = sum |A| |x| (in units of 2^(e + f)) is below the line
+// that the head of this file derives; columns whose x is zero wherever the row
+// has blocks are exact anyway. Lanes hold 16 columns and every second block each.
 template <int SRC>
-__device__ double stored_entry(const OzArgs& a, const OzSeg& g, long k, int part, int i, int j, int e) {
+__device__ __noinline__ uint32_t careful_columns(const OzArgs& a, const OzSeg& g, int row, int seg, int pass, int h) {
+  constexpr bool C = SRC != kDigits;
+  const int lane = threadIdx.x & 31, per = C ? 16 : a.nc, first = C ? 0 : 16 * h;
+  const int ncol = min(16, min(per, a.ncols - pass * per) - first), c = first + (lane & 15);
+  const int kb = g.row_ptr[row], ke = g.row_ptr[row + 1], ng = (a.B + 7) / 8;
+  bool care = a.fmax[(pass * a.nseg + seg) * 32 + c] == 2047;
+  if (a.care > 0.0f && kb < ke) {
+    float sum = 0.0f, most = 0.0f;
+    for (int k = kb + (lane >> 4); k < ke; k += 2) {
+      const float* nx = reinterpret_cast<const float*>(g.panels + (size_t)pass * a.pass_panels +
+                                                       (size_t)g.col[k] * a.panel + oz_norms_at(a.nc, a.nks)) + c;
+      const float* fl = g.floors + (long)k * ng;
+#pragma unroll 4
+      for (int q = 0; q < ng; ++q) {
+        float v = nx[q * a.nc];
+        if (C) v = 0.7071f * (v + nx[q * a.nc + 16]);  // at most the sum of the moduli
+        sum = fmaf(fl[q], v, sum);
+        most = fmaxf(most, v);
+      }
+    }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 16));
+    const float n = (float)(ke - kb) * (float)(a.B * (C ? 2 : 1));
+    const float roundings = (float)((ke - kb + a.chunk_blocks - 1) / a.chunk_blocks);  // of the fixed-point sum
+    const float line = a.care * (0.15f * rsqrtf(n) + roundings * exp2f((float)(39 - a.unit)) / n);
+    care |= !(sum >= line) && most > 0.0f;
+  }
+  return __ballot_sync(0xffffffffu, care) & ((1u << max(ncol, 0)) - 1u);
+}
+
+template <int SRC>
+__device__ __forceinline__ double stored_entry(const OzArgs& a, const OzSeg& g, long k, int part, int i, int j, int e) {
   const unsigned char* t = g.tiles + k * g.tstride;
   const long q = (long)j * a.B + i;
-  if constexpr (SRC == kDigits) return digit_value(t, a.B, i, j, e);
+  if constexpr (SRC == kDigits) return g.exact ? g.exact[k * g.exact_stride + q] : digit_value(t, a.B, i, j, e);
   else if constexpr (SRC == kF64C) return reinterpret_cast<const double*>(t)[2 * q + part];
   else {
     const float2 v = reinterpret_cast<const float2*>(t + (part ? g.im_off : 0))[q];
     return (double)v.x + (double)v.y;
   }
 }
+// Plain FP64 sums of block row `row` in the columns of mask (from col0 on), by a
+// whole CTA: a thread owns a row, four columns, which share the entries they
+// read, and every nsp-th block; the shares are added in order. Bound by the FP64
+// pipe, like the products that the digits replace.
 template <int SRC>
-__device__ __noinline__ double2 plain_entry(const OzArgs& a, const OzSeg& g, int row, int i, int col, int e) {
-  double re = 0.0, im = 0.0;
-  for (int k = g.row_ptr[row]; k < g.row_ptr[row + 1]; ++k)
-    for (int j = 0; j < a.B; ++j) {
-      const double ar = stored_entry<SRC>(a, g, k, 0, i, j, e);
-      const long xo = ((long)g.col[k] * a.B + j) * a.ldx + col;
-      if constexpr (SRC != kDigits) {
-        const double ai = stored_entry<SRC>(a, g, k, 1, i, j, e);
-        const double xr = g.x[2 * xo], xi = g.x[2 * xo + 1];
-        re = fma(ar, xr, fma(-ai, xi, re));
-        im = fma(ar, xi, fma(ai, xr, im));
-      } else {
-        re = fma(ar, g.x[xo], re);
+__device__ void plain_columns(const OzArgs& a, const OzSeg& g, int row, int col0, uint32_t mask, double* sums) {
+  constexpr bool C = SRC != kDigits;
+  constexpr int W = C ? 2 : 1;
+  const int kb = g.row_ptr[row], ke = g.row_ptr[row + 1], left = __popc(mask), nq = (left + 3) / 4;
+  for (int q0 = 0; q0 < nq; q0 += kOzThreads / a.B) {
+    const int nqs = min(nq - q0, kOzThreads / a.B), units = a.B * nqs, nsp = kOzThreads / units;
+    const int sp = threadIdx.x / units, unit = threadIdx.x - sp * units, i = unit % a.B, quad = q0 + unit / a.B;
+    int col[4];
+    double acc[4 * W];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) col[u] = col0 + __fns(mask, 0, min(4 * quad + u, left - 1) + 1);
+#pragma unroll
+    for (int u = 0; u < 4 * W; ++u) acc[u] = 0.0;
+    if (sp < nsp) {
+      const int e = SRC == kDigits ? g.rexp[(long)row * a.B + i] : 0;
+      for (int k = kb + sp; k < ke; k += nsp) {
+        const double* x = g.x + (long)g.col[k] * a.B * a.ldx * W;
+#pragma unroll 2
+        for (int j = 0; j < a.B; ++j, x += (long)a.ldx * W) {
+          const double ar = stored_entry<SRC>(a, g, k, 0, i, j, e);
+          if constexpr (C) {
+            const double ai = stored_entry<SRC>(a, g, k, 1, i, j, e);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const double2 v = reinterpret_cast<const double2*>(x)[col[u]];
+              acc[2 * u] = fma(ar, v.x, fma(-ai, v.y, acc[2 * u]));
+              acc[2 * u + 1] = fma(ar, v.y, fma(ai, v.x, acc[2 * u + 1]));
+            }
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc[u] = fma(ar, x[col[u]], acc[u]);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4 * W; ++u) sums[(sp * 4 * W + u) * units + unit] = acc[u];
+    }
+    __syncthreads();
+    if (sp == 0) {
+      double* y = g.y + ((long)row * a.B + i) * a.ldx * W;
+#pragma unroll
+      for (int u = 0; u < 4 * W; ++u) {
+        double v = 0.0;
+        for (int t = 0; t < nsp; ++t) v += sums[(t * 4 * W + u) * units + unit];
+        y[W * col[u / W] + u % W] = v;  // fewer than four columns: the last one again
       }
     }
-  return make_double2(re, im);
+    __syncthreads();
+  }
 }
 
 }  // namespace
 
 // Row exponents of FP64 blocks (column-major, complex interleaved): e[r B + i]
 // with |A_ij| <= 2^(e - 1) over block row r. A thread owns one row of the
-// blocks and a share of their columns.
+// blocks and a share of their columns. spread, if given: the most that the
+// exponents of a row's entries (complex: of the larger parts) differ, with its
+// own value.
 template <bool C>
 __global__ void k_oz_rows(const int* __restrict__ row_ptr, const double* __restrict__ blocks, long bstride, int B,
-                          int* __restrict__ e) {
-  __shared__ int top[128];
+                          int* __restrict__ e, int* spread) {
+  __shared__ int top[128], low[128];
   const int r = blockIdx.x, i = threadIdx.x % B, jg = threadIdx.x / B, nj = blockDim.x / B;
-  for (int t = threadIdx.x; t < B; t += blockDim.x) top[t] = 0;
+  for (int t = threadIdx.x; t < B; t += blockDim.x) {
+    top[t] = 0;
+    low[t] = 2047;
+  }
   __syncthreads();
-  int m = 0;
+  int m = 0, least = 2047;
   const int kb = row_ptr[r], ke = row_ptr[r + 1];
   for (int k = kb; k < ke; ++k)
     for (int j = jg; j < B; j += nj) {
       const long o = k * bstride + (long)j * B + i;
       if constexpr (C) {
         const double2 v = reinterpret_cast<const double2*>(blocks)[o];
-        m = max(m, max((__double2hiint(v.x) >> 20) & 0x7FF, (__double2hiint(v.y) >> 20) & 0x7FF));
+        const int be = max((__double2hiint(v.x) >> 20) & 0x7FF, (__double2hiint(v.y) >> 20) & 0x7FF);
+        m = max(m, be);
+        least = min(least, be);
       } else {
-        m = max(m, (__double2hiint(blocks[o]) >> 20) & 0x7FF);
+        const int be = (__double2hiint(blocks[o]) >> 20) & 0x7FF;
+        m = max(m, be);
+        least = min(least, be);
       }
     }
   atomicMax(&top[i], m);
+  atomicMin(&low[i], least);
   __syncthreads();
-  for (int t = threadIdx.x; t < B; t += blockDim.x) e[(long)r * B + t] = top[t] - 1021;
+  for (int t = threadIdx.x; t < B; t += blockDim.x) {
+    e[(long)r * B + t] = top[t] - 1021;
+    if (spread && kb < ke) atomicMax(spread, top[t] - low[t]);
+  }
+}
+
+// floors[k][q]: lower bounds of |A_ij| 2^-e_i (complex: of the larger part) over
+// columns 8 q .. 8 q + 7 and all rows of block k. A warp per group of columns.
+template <bool C>
+__global__ void k_oz_floors(const int* __restrict__ row_ptr, const double* __restrict__ blocks, long bstride, int B,
+                            const int* __restrict__ e, float* __restrict__ floors) {
+  const int r = blockIdx.x, ng = (B + 7) / 8, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int kb = row_ptr[r], n = (row_ptr[r + 1] - kb) * ng;
+  for (int u = threadIdx.x >> 5; u < n; u += nw) {
+    const long k = kb + u / ng;
+    const int j0 = 8 * (u % ng), nv = min(8, B - j0);
+    float m = FLT_MAX;
+    for (int i = lane; i < B; i += 32) {
+      const int ei = e[(long)r * B + i];
+      for (int c = 0; c < nv; ++c) {
+        const long o = k * bstride + (long)(j0 + c) * B + i;
+        if constexpr (C) {
+          const double2 v = reinterpret_cast<const double2*>(blocks)[o];
+          m = fminf(m, fmaxf(scaled_magnitude(v.x, ei), scaled_magnitude(v.y, ei)));
+        } else {
+          m = fminf(m, scaled_magnitude(blocks[o], ei));
+        }
+      }
+    }
+    const int bits = __reduce_min_sync(0xffffffffu, __float_as_int(m));  // not negative: ordered as integers
+    if (lane == 0) floors[k * ng + u % ng] = __int_as_float(bits);
+  }
 }
 
 // Digit bytes of real FP64 blocks (layout: group_bytes). A thread takes 8
@@ -616,8 +764,9 @@ __global__ void k_oz_cols(OzArgs a) {
 // Digit panels of x: cluster J of segment s at panels + pass a.pass_panels +
 // J panel; in it K chunk by K chunk, rows (t, c) (complex: [Re (t, c)] [Im (t,
 // c)]) K-major. A thread takes 8 consecutive source rows of one column;
-// columns and rows beyond the data get zeros. OWN: few rows, and every CTA
-// finds the column exponents itself instead of a launch (and a memset) before.
+// columns and rows beyond the data get zeros. It also writes their norm where
+// care is to be taken. OWN: few rows, and every CTA finds the column exponents
+// itself instead of a launch (and a memset) before.
 template <bool C, bool OWN>
 __global__ void k_oz_panels(OzArgs a) {
   __shared__ int red[32];
@@ -637,6 +786,7 @@ __global__ void k_oz_panels(OzArgs a) {
   const int half = C ? c >> 4 : 0, cc = C ? c & 15 : c;
   const bool live = col0 + cc < a.c0 + a.ncols;
   const int f = (OWN ? red[cc] : fmax[cc]) - 1021;
+  float norm = 0.0f;
   uint32_t w[8][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -646,6 +796,7 @@ __global__ void k_oz_panels(OzArgs a) {
       const long o = (J * a.B + j) * a.ldx + col0 + cc;
       v = C ? g.x[2 * o + half] : g.x[o];
     }
+    if (a.care > 0.0f) norm += scaled_magnitude(v, f);
     int d[8];
     oz_digits(v, f, d);
 #pragma unroll
@@ -657,8 +808,9 @@ __global__ void k_oz_panels(OzArgs a) {
   }
   const int chunk = kg / (2 * a.kw), kc = min(a.kw, a.nks - chunk * a.kw);
   const uint32_t sbo = (uint32_t)kc * 256u;
-  unsigned char* base = g.panels + (size_t)pass * a.pass_panels + (size_t)J * a.panel +
-                        (size_t)chunk * a.kw * a.nc * 8u * 32u + (uint32_t)(kg - chunk * 2 * a.kw) * 128u;
+  unsigned char* base = g.panels + (size_t)pass * a.pass_panels + (size_t)J * a.panel;
+  if (a.care > 0.0f) reinterpret_cast<float*>(base + oz_norms_at(a.nc, a.nks))[kg * a.nc + c] = norm;
+  base += (size_t)chunk * a.kw * a.nc * 8u * 32u + (uint32_t)(kg - chunk * 2 * a.kw) * 128u;
 #pragma unroll
   for (int s = 0; s < 8; ++s) {
     const int r = C ? half * 128 + s * 16 + cc : s * a.nc + c;
@@ -688,7 +840,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_bsr_oz(const __grid_constant_
   __shared__ uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_free[2], fin_bar;
   __shared__ uint64_t raw_full[kMaxRaws], raw_empty[kMaxRaws];
   __shared__ uint32_t tmem_slot;
-  __shared__ int abort_flag;
+  __shared__ int abort_flag, any_careful;
   volatile int* abort_v = &abort_flag;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int S = a.stages;
@@ -712,7 +864,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_bsr_oz(const __grid_constant_
       mbar_init(&acc_free[b], kEpiWarps);
     }
     mbar_init(&fin_bar, 1);
-    abort_flag = 0;
+    abort_flag = any_careful = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -960,6 +1112,12 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_bsr_oz(const __grid_constant_
       const int2 it = a.work ? __ldg(a.work + w) : make_int2(0, w);
       const OzSeg& g = a.seg[it.x];
       const int kb = __ldg(g.row_ptr + it.y), ke = __ldg(g.row_ptr + it.y + 1);
+      // looked up while the first accumulator fills
+      if (q == 0 && work && !(C && h)) {
+        const uint32_t m = careful_columns<SRC>(a, g, it.y, it.x, pass, h);
+        if (lane == 0) a.careful[2 * item + h] = (unsigned short)m;
+        if (m && lane == 0) any_careful = 1;
+      }
       long long P[16];
 #pragma unroll
       for (int c = 0; c < 16; ++c) P[c] = 0;
@@ -1009,32 +1167,31 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_bsr_oz(const __grid_constant_
       const int* f = a.fmax + (pass * a.nseg + it.x) * 32;
       const int e0 = kb < ke ? __ldg(g.rexp + (long)it.y * a.B + i) : 0, er = SRC == kPairsC ? max(e0, kMinPairExp) : e0;
       const long ro = ((long)it.y * a.B + i) * a.ldx + col0;
-      bool plain = false;  // a column with Inf or NaN
 #pragma unroll
       for (int c = 0; c < 16; ++c) {
         const int cc = C ? c : 16 * h + c;
         if (cc < ncol) {
-          const int fm = f[cc];
-          plain |= fm == 2047;
-          const double out = oz_to_double(P[c], er + (fm - 1021) - 14 - a.unit);
+          const double out = oz_to_double(P[c], er + (f[cc] - 1021) - 14 - a.unit);
           if (C) g.y[2 * (ro + cc) + h] = out;
           else g.y[ro + cc] = out;
         }
       }
-      if (plain)
-#pragma unroll 1
-        for (int cc = C ? 0 : 16 * h; cc < min(ncol, C ? 16 : 16 * h + 16); ++cc)
-          if (f[cc] == 2047) {
-            const double2 z = plain_entry<SRC>(a, g, it.y, i, col0 + cc, er);
-            if (C) g.y[2 * (ro + cc) + h] = h ? z.y : z.x;
-            else g.y[ro + cc] = z.x;
-          }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTmemCols));
+  // the block rows and columns that the digits do not serve, over what was written above
+  if (!any_careful || abort_flag) return;
+  for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
+    // halves 0 and 1 of the columns (complex: both halves hold the same ones; 16 columns: one half)
+    const uint32_t m = a.careful[2 * item] | (C || a.nc == 16 ? 0u : (uint32_t)a.careful[2 * item + 1] << 16);
+    if (!m) continue;
+    const int pass = item / a.nwork, w = item - pass * a.nwork;
+    const int2 it = a.work ? __ldg(a.work + w) : make_int2(0, w);
+    plain_columns<SRC>(a, a.seg[it.x], it.y, a.c0 + pass * (C ? 16 : a.nc), m, reinterpret_cast<double*>(smem));
+  }
 }
 
 bool bsr_oz_supported(int B, bool cplx, bool pairs, int max_row_blocks) {
@@ -1048,13 +1205,13 @@ size_t bsr_oz_panel_bytes(int B, bool cplx) {
 }
 
 cudaError_t launch_bsr_oz_rows(bool cplx, const int* row_ptr, const void* blocks, long bstride, int nrows, int B,
-                               int* rexp, cudaStream_t s) {
+                               int* rexp, int* spread, cudaStream_t s) {
   if (nrows == 0) return cudaSuccess;
   if (B < 1 || B > 128) return cudaErrorInvalidValue;
   const int threads = std::max(1, 384 / B) * B;
   const double* f = static_cast<const double*>(blocks);
-  if (cplx) k_oz_rows<true><<<nrows, threads, 0, s>>>(row_ptr, f, bstride, B, rexp);
-  else k_oz_rows<false><<<nrows, threads, 0, s>>>(row_ptr, f, bstride, B, rexp);
+  if (cplx) k_oz_rows<true><<<nrows, threads, 0, s>>>(row_ptr, f, bstride, B, rexp, spread);
+  else k_oz_rows<false><<<nrows, threads, 0, s>>>(row_ptr, f, bstride, B, rexp, spread);
   return cudaGetLastError();
 }
 cudaError_t launch_bsr_oz_tiles(const int* row_ptr, const double* blocks, long bstride, int nrows, int B,
@@ -1065,6 +1222,16 @@ cudaError_t launch_bsr_oz_tiles(const int* row_ptr, const double* blocks, long b
   const dim3 grid(nrows, (unsigned)std::min<long>(16, std::max<long>(1, (long)8 * 152 / nrows)));
   k_oz_tiles<<<grid, 256, 0, s>>>(row_ptr, blocks, bstride, B, rexp, static_cast<unsigned char*>(tiles),
                                   bsr_oz_tile_stride(B));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_bsr_oz_floors(bool cplx, const int* row_ptr, const void* blocks, long bstride, int nrows, int B,
+                                 const int* rexp, float* floors, cudaStream_t s) {
+  if (nrows == 0) return cudaSuccess;
+  if (B < 1 || B > 128) return cudaErrorInvalidValue;
+  const double* f = static_cast<const double*>(blocks);
+  if (cplx) k_oz_floors<true><<<nrows, 512, 0, s>>>(row_ptr, f, bstride, B, rexp, floors);
+  else k_oz_floors<false><<<nrows, 512, 0, s>>>(row_ptr, f, bstride, B, rexp, floors);
   return cudaGetLastError();
 }
 

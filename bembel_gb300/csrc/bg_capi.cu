@@ -532,8 +532,8 @@ static bg_status upload_tables(bg_operator* op) {
         BG_CHECK(op->d_far_work_alt[o - 1].upload(alt, s), "far-field work list");
       }
   }
-  BG_CHECK(op->d_err.alloc(sizeof(int)), "error flag");
-  BG_CHECK(cudaMemsetAsync(op->d_err.p, 0, sizeof(int), s), "error flag");
+  BG_CHECK(op->d_err.alloc(2 * sizeof(int)), "error flag");  // and the far field's spread
+  BG_CHECK(cudaMemsetAsync(op->d_err.p, 0, 2 * sizeof(int), s), "error flag");
   BG_CHECK(cudaStreamSynchronize(s), "upload tables");
   return BG_OK;
 }
@@ -706,9 +706,9 @@ extern "C" bg_status bg_operator_memory(const bg_operator* op, size_t* allocated
   size_t e = (size_t)op->dense.col.size() * op->block_stride(op->dense.B) * sb +
              (size_t)op->dense.col.size() * op->block_stride32(op->dense.B) * sb / 2;
   if (!op->cplx) e += (size_t)op->dense.col.size() * op->block_stride(op->dense.B) * sizeof(float2);  // double-float
-  if (op->near_oz)  // digit bytes, row exponents, x digit panels
+  if (op->near_oz)  // digit bytes, row exponents and floors, x digit panels
     e += (op->cplx ? 0 : op->digit_bytes((long)op->dense.col.size(), op->dense.B)) +
-         (size_t)op->dense.nrows * op->dense.B * sizeof(int) + (size_t)op->dense.nrows * bsr_oz_panel_bytes(op->dense.B, op->cplx) * oz_passes(op, op->dense.nrows, 32);
+         op->near_tail() + (size_t)op->dense.nrows * bsr_oz_panel_bytes(op->dense.B, op->cplx) * oz_passes(op, op->dense.nrows, 32);
   for (int l = 0; l <= op->leaf_level && l < (int)op->far.size(); ++l) {
     const size_t nb = op->far[l].col.size();
     const size_t ncl = (size_t)op->nclusters(l);
@@ -866,6 +866,9 @@ static OzSeg oz_near_seg(const bg_operator* op, const DevBuf& dense64, const Dev
   g.tstride = op->cplx ? op->block_stride(f.B) * 16 : bsr_oz_tile_stride(f.B);
   g.rexp = reinterpret_cast<const int*>(dig.as<unsigned char>() +
                                         (op->cplx ? 0 : op->digit_bytes((long)f.col.size(), f.B)));
+  g.floors = reinterpret_cast<const float*>(g.rexp + (size_t)f.nrows * f.B);
+  g.exact = dense64.as<double>();
+  g.exact_stride = op->block_stride(f.B);
   g.ncl = f.nrows;
   g.x = op->w_xss.as<double>();
   g.y = op->w_yss.as<double>();
@@ -873,19 +876,29 @@ static OzSeg oz_near_seg(const bg_operator* op, const DevBuf& dense64, const Dev
   return g;
 }
 // row exponents of segment f (FP64 blocks) and, for real operators, digit
-// bytes into dig, the exponents behind ahead bytes
-static cudaError_t build_digits(bg_operator* op, const BsrSegment& f, const void* blocks, DevBuf* dig, size_t ahead) {
-  cudaError_t e = dig->alloc(ahead + (size_t)f.nrows * f.B * sizeof(int));
+// bytes into dig, the exponents behind ahead bytes; tail: bytes for what
+// follows, spread as in launch_bsr_oz_rows
+static cudaError_t build_digits(bg_operator* op, const BsrSegment& f, const void* blocks, DevBuf* dig, size_t ahead,
+                                size_t tail, int* spread) {
+  cudaError_t e = dig->alloc(ahead + tail);
   if (e != cudaSuccess) return e;
   unsigned char* t = dig->as<unsigned char>();
   int* rexp = reinterpret_cast<int*>(t + ahead);
   cudaStream_t s = op->ctx->stream;
   const long bs = op->block_stride(f.B);
-  e = launch_bsr_oz_rows(op->cplx, f.d_row_ptr.as<int>(), blocks, bs, f.nrows, f.B, rexp, s);
+  e = launch_bsr_oz_rows(op->cplx, f.d_row_ptr.as<int>(), blocks, bs, f.nrows, f.B, rexp, spread, s);
   if (e == cudaSuccess && !op->cplx)
     e = launch_bsr_oz_tiles(f.d_row_ptr.as<int>(), static_cast<const double*>(blocks), bs, f.nrows, f.B, rexp, t, s);
   return e;
 }
+
+// The most that the exponents of one row of far-field couplings may differ for
+// the digits: their error is relative to the row's largest coupling, that of
+// the double-float product to each one (bg_bsr_oz.cu). The spheres and the
+// torus have 5 (Laplace, and Helmholtz at real wavenumbers); a wavenumber with
+// an imaginary part spreads the couplings exponentially, a patch that shrinks
+// to a point as far as its surface measure.
+constexpr int kFarSpread = 10;
 
 static bg_status assemble_far(bg_operator* op) {
   cudaStream_t s = op->ctx->stream;
@@ -899,6 +912,9 @@ static bg_status assemble_far(bg_operator* op) {
   }
   op->far_tiles = false;
   if (!any_far) return BG_OK;
+  if (op->cplx) op->far_wide = false;  // the wavenumber's; a real operator's geometry stays
+  int* spread = op->far_oz && !op->far_wide ? op->d_err.as<int>() + 1 : nullptr;
+  if (spread) BG_CHECK(cudaMemsetAsync(spread, 0, sizeof(int), s), "far-field spread");
   for (int l = 0; l <= op->leaf_level; ++l) {
     if ((int)op->d_pts64.size() <= l) {
       op->d_pts64.push_back(new DevBuf());
@@ -943,7 +959,8 @@ static bg_status assemble_far(bg_operator* op) {
       // double-float pairs of Re and Im for the complex FP64 product
       const long sdf = ((long)f.B * f.B + 1) / 2 * 2;
       const size_t ahead = op->digit_bytes((long)f.col.size(), f.B);
-      if (op->far_oz) BG_CHECK(build_digits(op, f, op->d_far64[l]->p, op->d_far_df[l], ahead), "far-field exponents");
+      if (op->far_oz) BG_CHECK(build_digits(op, f, op->d_far64[l]->p, op->d_far_df[l], ahead,
+                                            (size_t)f.nrows * f.B * sizeof(int), spread), "far-field exponents");
       else BG_CHECK(op->d_far_df[l]->alloc(ahead), "far field storage");
       BG_CHECK(launch_split_df_cplx_blocks(op->d_far64[l]->p, op->block_stride(f.B), (long)f.B * f.B, (long)f.col.size(),
                                            sdf, op->d_far_df[l]->p, s),
@@ -961,7 +978,8 @@ static bg_status assemble_far(bg_operator* op) {
     } else {
       // digits, or (hi, lo) FP32 pairs, of the same blocks for the FP64 product
       if (op->far_digits())
-        BG_CHECK(build_digits(op, f, op->d_far64[l]->p, op->d_far_df[l], op->digit_bytes((long)f.col.size(), f.B)),
+        BG_CHECK(build_digits(op, f, op->d_far64[l]->p, op->d_far_df[l], op->digit_bytes((long)f.col.size(), f.B),
+                              (size_t)f.nrows * f.B * sizeof(int), spread),
                  "far-field digits");
       else BG_CHECK(op->d_far_df[l]->alloc(bytes), "far field storage");
       if (!op->far_digits())
@@ -981,6 +999,15 @@ static bg_status assemble_far(bg_operator* op) {
     BG_CHECK(cudaStreamSynchronize(s), "far-field assembly");
     // the products read the digits (or pairs) and the tiles, not the FP64 blocks
     if (!op->keep_far64 && op->d_far_df[l]->p) op->d_far64[l]->release();
+  }
+  if (spread && op->store_far) {
+    int most = 0;
+    BG_CHECK(cudaMemcpy(&most, spread, sizeof(int), cudaMemcpyDeviceToHost), "far-field spread");
+    if (most > kFarSpread) {
+      op->far_wide = true;
+      op->cap = 0;  // other work vectors
+      if (!op->cplx) return assemble_far(op);  // the couplings again, as pairs
+    }
   }
   op->far_tiles = tiled_levels == far_levels && op->leaf_level < kMaxFarLevels;
   return BG_OK;
@@ -1439,6 +1466,7 @@ extern "C" bg_status bg_operator_assemble_wavenumbers(bg_operator* op) {
     std::swap(slot.atiles, op->d_far_atiles);
     std::swap(slot.ainv, op->d_far_ainv);
     slot.far_tiles = op->far_tiles;
+    slot.far_wide = op->far_wide;
     fresh_far_fields(op);
     // the prepared copy of this near field is no longer needed
     for (size_t i = 0; i < op->near_cache.size(); ++i)
@@ -1534,7 +1562,12 @@ extern "C" bg_status bg_operator_assemble(bg_operator* op) {
     // digits (complex: row exponents) of the blocks for the FP64-accurate tensor-core product
     if (nb > 0 && op->near_oz) {
       e = build_digits(op, op->dense, op->d_dense64.p, &op->d_dense_dig,
-                       op->cplx ? 0 : op->digit_bytes(nb, (int)B));
+                       op->cplx ? 0 : op->digit_bytes(nb, (int)B), op->near_tail(), nullptr);
+      if (e == cudaSuccess) {
+        const OzSeg g = oz_near_seg(op, op->d_dense64, op->d_dense_dig);
+        e = launch_bsr_oz_floors(op->cplx, g.row_ptr, op->d_dense64.p, op->block_stride((int)B), op->dense.nrows, (int)B,
+                                 g.rexp, const_cast<float*>(g.floors), op->ctx->stream);
+      }
       if (e == cudaSuccess) e = cudaStreamSynchronize(op->ctx->stream);
       if ((st = cuda_status(op->ctx, e, "near-field digits")) != BG_OK) return st;
     }
@@ -1548,6 +1581,10 @@ extern "C" bg_status bg_operator_assemble(bg_operator* op) {
 }
 
 // ---------------------------------------------------------------------------
+// bytes of a block row's marks for one pass of the FP64-accurate tensor-core
+// product; with those of the panel of a column cluster
+constexpr size_t kOzMarks = 2 * sizeof(unsigned short);
+static size_t oz_scratch(int B, bool cplx) { return bsr_oz_panel_bytes(B, cplx) + kOzMarks; }
 // bytes of one pass of the far field's digit panels; off: the levels' offsets in it
 static size_t oz_far_panels(const bg_operator* op, size_t* off) {
   size_t n = 0;
@@ -1571,7 +1608,7 @@ static bool near_by_digits(const bg_operator* op, const DevBuf& dig, int nc, boo
 // columns c0 .. c0 + nc - 1 (rows of ld scalars) of the near field
 constexpr int kOzFmax = 2 * kOzMaxSegs * 32;
 static cudaError_t oz_near_product(const bg_operator* op, const DevBuf& dense64, const DevBuf& dig, int ld, int c0, int nc,
-                                   cudaStream_t s) {
+                                   bool mixed, cudaStream_t s) {
   OzArgs a{};
   a.seg[0] = oz_near_seg(op, dense64, dig);
   a.nseg = 1;
@@ -1583,6 +1620,8 @@ static cudaError_t oz_near_product(const bg_operator* op, const DevBuf& dense64,
   a.pass_panels = (size_t)op->dense.nrows * bsr_oz_panel_bytes(a.B, op->cplx);
   a.fmax = op->w_oz_fmax.as<int>() + kOzFmax;  // the far field has the first half and may run beside
   a.err = op->d_err.as<int>();
+  a.care = mixed && !op->cplx ? 0.0f : 1.0f;  // the mixed real product's far field is in FP32 anyway
+  a.careful = reinterpret_cast<unsigned short*>(op->w_oz_near.as<unsigned char>() + a.pass_panels * op->oz_near_passes);
   return launch_bsr_oz(op->cplx, false, a, op->near_row_max, op->oz_near_passes, s);
 }
 // the far field of every level with couplings df, y[l] to z[l]
@@ -1602,6 +1641,7 @@ static cudaError_t oz_far_product(const bg_operator* op, const std::vector<DevBu
   a.ncols = nc;
   a.fmax = op->w_oz_fmax.as<int>();
   a.err = op->d_err.as<int>();
+  a.careful = reinterpret_cast<unsigned short*>(op->w_oz_far.as<unsigned char>() + a.pass_panels * op->oz_far_passes);
   return launch_bsr_oz(op->cplx, op->cplx, a, op->far_row_max, op->oz_far_passes, op->ctx->stream);
 }
 
@@ -1630,7 +1670,7 @@ bg_status ensure_work(bg_operator* op, int nrhs) {
     BG_CHECK(op->w_y[l]->alloc(n), "work vectors");
     BG_CHECK(op->w_z[l]->alloc(n), "work vectors");
     // double-float split of y (complex: 16 columns at a time)
-    if (!op->far_oz || op->maxwell())
+    if (!op->far_oz || op->any_far_wide() || op->maxwell())
       BG_CHECK(op->w_ydf[l]->alloc(op->cplx ? (size_t)op->nclusters(l) * op->np * op->np * 32 * sizeof(float2) : n),
                "work vectors");
     const size_t tb = op->cplx ? far_h16c_btile_bytes(op->np * op->np) : far_h16_btile_bytes(op->np * op->np);
@@ -1644,15 +1684,18 @@ bg_status ensure_work(bg_operator* op, int nrhs) {
       BG_CHECK(op->w_binv[l]->alloc(sizeof(float) * 32 * op->nclusters(l)), "work vectors");
     }
   }
-  // digit panels of x for the FP64-accurate tensor-core products
+  // digit panels of x for the FP64-accurate tensor-core products, and behind
+  // them the marks of every block row
   {
     op->oz_near_passes = oz_passes(op, op->dense.nrows, nrhs);
     if (op->near_oz)
-      BG_CHECK(op->w_oz_near.alloc((size_t)op->dense.nrows * bsr_oz_panel_bytes(op->dense.B, op->cplx) * op->oz_near_passes),
+      BG_CHECK(op->w_oz_near.alloc((size_t)op->dense.nrows * oz_scratch(op->dense.B, op->cplx) * op->oz_near_passes),
                "work vectors");
     const int cols = op->maxwell() ? 4 * std::min(nrhs, (int)bg_operator::kMwRhsChunk) : nrhs;
     op->oz_far_passes = oz_passes(op, op->n_far_work, cols);
-    if (op->far_oz) BG_CHECK(op->w_oz_far.alloc(oz_far_panels(op, nullptr) * op->oz_far_passes), "work vectors");
+    if (op->far_oz)
+      BG_CHECK(op->w_oz_far.alloc((oz_far_panels(op, nullptr) + (size_t)op->n_far_work * kOzMarks) * op->oz_far_passes),
+               "work vectors");
     BG_CHECK(op->w_oz_fmax.alloc((size_t)2 * kOzFmax * sizeof(int)), "work vectors");
   }
   if (op->fmm_fused) {
@@ -1741,7 +1784,7 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver, 
     for (int q = 0; q < nk; ++q) {
       const bg_operator::KSlot& k = op->kslots[q];
       if (!near32 && near_by_digits(op, k.dense_dig, nr, solver)) {
-        BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return oz_near_product(op, k.dense64, k.dense_dig, nrhs, q * nr, nr, s); }),
+        BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return oz_near_product(op, k.dense64, k.dense_dig, nrhs, q * nr, nr, mixed, s); }),
                  "near-field product (batched wavenumbers, tensor cores)");
         continue;
       }
@@ -1766,7 +1809,7 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver, 
   } else if ((!mixed || pl.mixed_near == 0) && near_by_digits(op, op->d_dense_dig, nrhs, solver)) {
     // FP64-accurate near field on the tensor cores: 8 integer digits of 7
     // bits per operand, exact integer accumulation, one rounding at the end
-    BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return oz_near_product(op, op->d_dense64, op->d_dense_dig, nrhs, 0, nrhs, sn); }),
+    BG_CHECK(timed_launch(op->ctx, KC_NEAR, [&] { return oz_near_product(op, op->d_dense64, op->d_dense_dig, nrhs, 0, nrhs, mixed, sn); }),
              "near-field product (tensor cores, integer digits)");
   } else if (mixed && !op->cplx && op->d_dense_df.p && (pl.mixed_near != 0 || !op->near_oz)) {
     // FP64-accurate near field in double-float: blocks and x as FP32 (hi, lo)
@@ -2019,7 +2062,7 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver, 
       return BG_OK;
     };
     // FP64 far field on the tensor cores, all levels in one launch
-    const bool oz_far = !mixed && op->far_oz && op->store_far && !(solver && op->maxwell());
+    const bool oz_far = !mixed && op->far_oz && !op->any_far_wide() && op->store_far && !(solver && op->maxwell());
     if (oz_far && op->maxwell()) {
       const std::complex<double> kap(op->kre, op->kim), mk2 = -1.0 / (kap * kap);
       for (int r0 = 0; r0 < nrhs; r0 += bg_operator::kMwRhsChunk) {

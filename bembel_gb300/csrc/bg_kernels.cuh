@@ -228,6 +228,9 @@ struct OzSeg {
   const unsigned char* tiles;  // block k at + k tstride bytes (pairs of Im: im_off bytes further)
   long tstride, im_off;
   const int* rexp;             // row exponents [rows][B]
+  const float* floors;         // care: [blocks][ceil(B / 8)], lower bounds of |A_ij| 2^-e_i over 8 columns, all rows
+  const double* exact;         // digit bytes: the FP64 blocks they came from, exact_stride apart; nullptr: not kept
+  long exact_stride;
   const double* x;             // [ncl B][ldx] (complex interleaved)
   double* y;                   // [rows B][ldx], written
   unsigned char* panels;       // scratch, bsr_oz_panel_bytes per cluster and pass (those of pass p at + p pass_panels)
@@ -242,6 +245,10 @@ struct OzArgs {
   size_t pass_panels;
   int* fmax;           // scratch, 32 ints per segment and pass
   int* err;
+  // 1: entries whose digits may lose more than FP64 sums are summed in FP64
+  // (needs the floors); 0: never
+  float care;
+  unsigned short* careful;  // scratch, two per block row and pass: the columns concerned
   // set by the launcher
   int nitems, unit, rg, nks, kw, nch, bps, nc, stages, raws, chunk_blocks;
   uint32_t slice, stage, raw, raw_off, panel, tstride;
@@ -250,11 +257,15 @@ struct OzArgs {
 bool bsr_oz_supported(int B, bool cplx, bool pairs, int max_row_blocks);
 size_t bsr_oz_panel_bytes(int B, bool cplx);  // 0: block size not supported
 long bsr_oz_tile_stride(int B);               // bytes between the (real) blocks' digit bytes
-// row exponents [nrows B] of FP64 blocks (column-major, complex interleaved), digit bytes of real ones
+// row exponents [nrows B] of FP64 blocks (column-major, complex interleaved), digit bytes of real ones; spread, if
+// given, becomes the most that exponents differ within a row, or stays
 cudaError_t launch_bsr_oz_rows(bool cplx, const int* row_ptr, const void* blocks, long bstride, int nrows, int B,
-                               int* rexp, cudaStream_t s);
+                               int* rexp, int* spread, cudaStream_t s);
 cudaError_t launch_bsr_oz_tiles(const int* row_ptr, const double* blocks, long bstride, int nrows, int B,
                                 const int* rexp, void* tiles, cudaStream_t s);
+// floors of the blocks (OzSeg)
+cudaError_t launch_bsr_oz_floors(bool cplx, const int* row_ptr, const void* blocks, long bstride, int nrows, int B,
+                                 const int* rexp, float* floors, cudaStream_t s);
 // cplx: complex pairs (pairs set) or FP64, else digit bytes; max_row_blocks as
 // bsr_oz_supported, over the segments; max_passes: passes of 32 columns
 // (complex: 16) the panel scratch has room for

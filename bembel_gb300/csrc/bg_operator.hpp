@@ -163,7 +163,7 @@ struct bg_operator {
     double kre = 0.0, kim = 0.0;
     DevBuf dense64, dense32, dense_dig;
     std::vector<DevBuf*> far64, far_df, atiles, ainv;
-    bool far_tiles = false;
+    bool far_tiles = false, far_wide = false;
   };
   std::vector<KSlot> kslots;
   int kslot_active = -1;
@@ -188,6 +188,7 @@ struct bg_operator {
     std::swap(d_far_atiles, k.atiles);
     std::swap(d_far_ainv, k.ainv);
     std::swap(far_tiles, k.far_tiles);
+    std::swap(far_wide, k.far_wide);
   }
   void activate_slot(int q) {
     if (q == kslot_active) return;
@@ -219,7 +220,7 @@ struct bg_operator {
   std::vector<DevBuf*> d_tan64, d_tan32;             // per level, Maxwell: tangents dx, dy of every point
   DevBuf d_dense64;                       // dense blocks (FP64)
   DevBuf d_dense_dig;                     // near_oz operators: their digit bytes (real; bg_bsr_oz.cu), then their
-                                          // row exponents
+                                          // row exponents and floors
   DevBuf d_dense32;                       // FP32 copy of the dense blocks (BG_PREC_FP32)
   DevBuf d_dense_df;                      // real operators: FP32 (hi, lo) pairs of the dense blocks, the
                                           // near field of BG_PREC_MIXED products (double-float, FP64 accuracy)
@@ -235,9 +236,15 @@ struct bg_operator {
                                           // Im); with far_oz the row exponents behind them
   // FP64-accurate products on the tensor cores (bg_bsr_oz.cu) for the far and
   // the near field, fixed by the block sizes and rows when the operator is
-  // created
-  bool far_oz = false, near_oz = false;
-  bool far_digits() const { return far_oz && !cplx; }
+  // created; far_wide: the couplings assembled spread too far within a row
+  // for digits (kFarSpread) and take the double-float product
+  bool far_oz = false, near_oz = false, far_wide = false;
+  bool any_far_wide() const {  // this wavenumber's or a batched one's
+    bool w = far_wide;
+    for (const auto& k : kslots) w |= k.far_wide;
+    return w;
+  }
+  bool far_digits() const { return far_oz && !cplx && !far_wide; }
   std::vector<DevBuf*> d_far_atiles;      // per level: FP16 hi/lo tensor-core tiles of the low-rank blocks
   std::vector<DevBuf*> d_far_ainv;        // per level: inverse power-of-two scale of every tile
   bool far_tiles = false;                 // every far-field level has its tiles
@@ -335,6 +342,10 @@ struct bg_operator {
   size_t digit_bytes(long nblocks, int B) const {
     const long s = ((long)B * B + 1) / 2 * 2 * 8;
     return (size_t)nblocks * s * (cplx ? 2 : 1);
+  }
+  // bytes of the near field's row exponents and floors, which follow them
+  size_t near_tail() const {
+    return (size_t)dense.nrows * dense.B * sizeof(int) + dense.col.size() * (size_t)((dense.B + 7) / 8) * sizeof(float);
   }
   int stype(bool fp32) const { return (fp32 ? 2 : 0) + (cplx ? 1 : 0); }
   // Maxwell: the far field is stored as the scalar kernel matrix of each

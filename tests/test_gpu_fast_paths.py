@@ -206,3 +206,130 @@ def test_transforms_of_large_panels(ctx, oracle, P, np_, mcl, kind):
         for prec, tol in (("fp64", FP64_TOL), ("mixed", 1e-4), ("fp32", 1e-4))[:1 if np_ == 12 else 3]:
             y = A.matvec(x[:, :n], precision=prec)
             assert np.linalg.norm(y - ref[:, :n]) < tol * np.linalg.norm(ref[:, :n]), (n, prec)
+
+
+def _spread_columns(d, T, rng, cplx):
+    """Columns whose entries differ widely: single unknowns, magnitudes from 1
+    to 1e-20 at random and by position, beside a normal one."""
+    N = d.N
+    x = np.zeros((N, 8), dtype=complex if cplx else float)
+    for c, j in enumerate((0, N // 3, N - 1)):
+        x[j, c] = 1.0
+    x[:, 3] = rng.normal(size=N) * 10.0 ** (-20 * rng.uniform(size=N))
+    x[:, 4] = rng.normal(size=N) * 10.0 ** (-20 * np.arange(N) / N)
+    x[:, 5] = rng.normal(size=N) * np.where(np.arange(N) < N // 6, 1.0, 1e-18)
+    x[:, 6] = rng.normal(size=N) * np.where(np.arange(N) == N // 2, 1e30, 1.0)
+    x[:, 7] = rng.normal(size=N)
+    if cplx:
+        x[:, 3:] *= np.exp(1j * rng.uniform(0, 2 * np.pi, (N, 5)))
+    return x
+
+
+@pytest.mark.parametrize("geo,P,kind,kappa", [(SPHERE, 0, 0, 0), (SPHERE, 1, 0, 0), (SPHERE, 2, 0, 0), (SPHERE, 1, 1, 2.0),
+                                              (SPHERE, 1, 1, 2.0 - 30.0j), (TORUS, 2, 1, 1.0 - 20.0j)])
+def test_digit_near_field_keeps_every_entry(ctx, geo, P, kind, kappa):
+    """Entry by entry the FP64 product is as good as plain FP64 sums, whatever
+    the sizes of x in one column and of the blocks in one row (a damped kernel
+    decays by up to e^-120 over the surface): the error of each entry is below
+    the bound of such sums, (n + 20) 2^-53 times |T^t| |A| |T| |x| for rows of
+    n = S terms (complex: 2 n, and twice that for the two parts), against sums
+    in extended precision. The 20 covers T and T^t (at most 16 terms a row)."""
+    d = _operator(ctx, geo, 1, P, kind, kappa)
+    assert d.n_lowrank == 0
+    T, A = _fp64_dense(d)
+    x = _spread_columns(d, T, np.random.default_rng(15), bool(kind))
+    wide = np.clongdouble if kind else np.longdouble
+    Tw = T.astype(np.longdouble)
+    ref = Tw.T @ (A.astype(wide) @ (Tw @ x.astype(wide)))
+    bound = np.abs(T).T @ (np.abs(A) @ (np.abs(T) @ np.abs(x)))
+    n = d.S * (2 if kind else 1)
+    for prec in ("fp64", "mixed") if kind else ("fp64",):  # the real mixed product promises less
+        y = d.get_discrete_operator().matvec(x, precision=prec)
+        err = np.abs(y - ref).astype(float)
+        assert (err <= (2 if kind else 1) * (n + 20) * 2.0 ** -53 * bound).all(), \
+            (prec, (err / np.maximum(bound, 1e-300)).max(axis=0))
+
+
+@pytest.mark.parametrize("M,P,kind,kappa,np_", [(2, 1, 0, 0, 6), (3, 1, 0, 0, 9), (2, 2, 1, 2.0, 9), (2, 1, 1, 2.0 - 1.0j, 7)])
+def test_digit_far_field_keeps_every_entry(ctx, oracle, M, P, kind, kappa, np_):
+    """With a far field, entry by entry the FP64 product stays within n 2^-48
+    |T^t| |A| |T| |x| (n = S, the bound of double-float sums over a row; A the
+    dense matrix) of the oracle's FP64 product of the same H2 matrix, for
+    columns of widely different sizes."""
+    d = _operator(ctx, SPHERE, M, P, kind, kappa, np_)
+    assert d.n_lowrank > 0
+    o = oracle.Problem(SPHERE, M, P, kind, kappa=kappa, np_=np_)
+    T = o.transform_dense()
+    x = _spread_columns(d, T, np.random.default_rng(18), bool(kind))
+    bound = np.abs(T).T @ (np.abs(o.dense_ss()) @ (np.abs(T) @ np.abs(x)))
+    err = np.abs(d.get_discrete_operator().matvec(x) - o.matvec(x))
+    assert (err <= d.S * 2.0 ** -48 * bound).all(), (err / bound).max(axis=0)
+
+
+@pytest.mark.parametrize("np_", [6, 9])
+@pytest.mark.parametrize("batched", [False, True])
+def test_far_field_of_a_damped_kernel(ctx, oracle, np_, batched):
+    """A column that lives on one side of the surface, with a kernel that
+    decays by e^-28 to the other side: the values there, 1e-8 to 1e-12 of the
+    largest, match the oracle to 1e-10 of themselves, by itself and as one of
+    two batched wavenumbers (the other without damping)."""
+    kappa = 1.5 - 14.0j
+    d = _operator(ctx, SPHERE, 3, 1, 1, 1.5, np_)
+    if batched:
+        d.prepare_wavenumbers([1.5, kappa])
+        d.assemble_wavenumbers()
+    else:
+        d.get_discrete_operator().matvec(np.ones(d.N))  # work vectors of the undamped operator
+        d.lin_op.set_wavenumber(kappa)
+        d.compute()
+    o = oracle.Problem(SPHERE, 3, 1, 1, kappa=kappa, np_=np_)
+    rng = np.random.default_rng(16)
+    x = np.zeros((d.N, 4), dtype=complex)
+    x[:d.N // 24] = rng.uniform(0.5, 1.0, (d.N // 24, 4))
+    ref = o.matvec(x)
+    y = d.get_discrete_operator().matvec(np.hstack([x, x]) if batched else x)[:, -4:]
+    size = np.linalg.norm(ref, axis=1)
+    low = size < 1e-8 * size.max()
+    assert low.sum() > d.N // 20
+    assert (np.linalg.norm(y - ref, axis=1)[low] < 1e-10 * size[low]).all()
+
+
+DEGENERATE_DAT = """# nurbs mesh v.2.1
+# screen
+# a square whose upper side is shrunk to nearly a point
+#
+2 3 1 0 0
+PATCH 0
+1 1
+2 2
+0 0 1 1
+0 0 1 1
+0 1 0 0.000001
+0 0 1 1
+0 0 0 0
+1 1 1 1
+"""
+
+
+def test_far_field_of_a_shrunk_patch(ctx, oracle, tmp_path):
+    """Couplings of one row that differ by the surface measure of a nearly
+    singular patch (1e-6 at the shrunk side) are kept as FP32 pairs instead of
+    digits: unit vectors there and normal columns match the oracle, 1e-12 of
+    the column, for one column and several, also after another assembly."""
+    geo = str(tmp_path / "shrunk.dat")
+    with open(geo, "w") as f:
+        f.write(DEGENERATE_DAT)
+    d = _operator(ctx, geo, 4, 1, 0, 0.0, 9)
+    assert d.n_lowrank > 0
+    o = oracle.Problem(geo, 4, 1, 0, np_=9)
+    rng = np.random.default_rng(17)
+    x = rng.normal(size=(d.N, 33))
+    x[:, 0] = 0.0
+    x[-1, 0] = 1.0
+    ref = o.matvec(x)
+    A = d.get_discrete_operator()
+    for _ in range(2):
+        for n in (1, 5, 33):
+            y = A.matvec(x[:, :n])
+            assert (np.linalg.norm(y - ref[:, :n], axis=0) < FP64_TOL * np.linalg.norm(ref[:, :n], axis=0)).all(), n
+        d.compute()
