@@ -897,7 +897,7 @@ static cudaError_t build_digits(bg_operator* op, const BsrSegment& f, const void
 // the double-float product to each one (bg_bsr_oz.cu). The spheres and the
 // torus have 5 (Laplace, and Helmholtz at real wavenumbers); a wavenumber with
 // an imaginary part spreads the couplings exponentially, a patch that shrinks
-// to a point as far as its surface measure.
+// to a point as far as its surface measure. Couplings with Inf or NaN pass any line.
 constexpr int kFarSpread = 10;
 
 static bg_status assemble_far(bg_operator* op) {

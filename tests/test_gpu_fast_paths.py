@@ -333,3 +333,53 @@ def test_far_field_of_a_shrunk_patch(ctx, oracle, tmp_path):
             y = A.matvec(x[:, :n])
             assert (np.linalg.norm(y - ref[:, :n], axis=0) < FP64_TOL * np.linalg.norm(ref[:, :n], axis=0)).all(), n
         d.compute()
+
+
+LARGE_DAT = """# nurbs mesh v.2.1
+# screen
+# a square of side 1e150, whose surface measure is beyond FP64
+#
+2 3 1 0 0
+PATCH 0
+1 1
+2 2
+0 0 1 1
+0 0 1 1
+0 1e150 0 1e150
+0 0 1e150 1e150
+0 0 0 0
+1 1 1 1
+"""
+
+
+@pytest.mark.parametrize("geo,M,kind,kappa,np_", [
+    (None, 1, 0, 0.0, 6), (SPHERE, 1, 1, np.nan, 6), (SPHERE, 1, 1, 1.0 + 800.0j, 6), (SPHERE, 3, 1, np.nan, 6),
+    (SPHERE, 3, 1, 1.0 + 60.0j, 9), (SPHERE, 3, 1, 1.0 + 800.0j, 7), (SPHERE, 2, 2, np.nan, 6)])
+def test_operators_with_infinities(ctx, tmp_path, geo, M, kind, kappa, np_):
+    """Where every row of the couplings has Inf or NaN (a surface measure or a
+    growing kernel beyond FP64, a wavenumber that is NaN), no entry of the
+    product is finite, at any number of columns. Growth by e^120 leaves FP64
+    couplings finite but passes the range of the FP32 pairs that complex far
+    fields are kept as: not finite there either. With a finite wavenumber again
+    the operator is the one it was before (1e-13)."""
+    if geo is None:
+        geo = str(tmp_path / "large.dat")
+        with open(geo, "w") as f:
+            f.write(LARGE_DAT)
+    d = _operator(ctx, geo, M, 1, kind, 2.0, np_)
+    rng = np.random.default_rng(19)
+    x = rng.normal(size=(d.N, 17)) + (1j * rng.normal(size=(d.N, 17)) if kind else 0)
+    if kind:
+        clean = d.get_discrete_operator().matvec(x)
+        d.lin_op.set_wavenumber(kappa)
+        d.compute()
+    A = d.get_discrete_operator()
+    near = d.n_lowrank == 0 or np.isnan(kappa)  # the near field, which "mixed" keeps in FP64, has them too
+    for n in (1, 2, 3, 5, 17):
+        for prec in ("fp64", "mixed") if near else ("fp64",):
+            assert not np.isfinite(A.matvec(x[:, :n], precision=prec)).any(), (n, prec)
+    if kind:
+        d.lin_op.set_wavenumber(2.0)
+        d.compute()
+        y = d.get_discrete_operator().matvec(x)
+        assert np.linalg.norm(y - clean) < 1e-13 * np.linalg.norm(clean)
