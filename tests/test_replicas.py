@@ -92,3 +92,17 @@ def test_bench_column_errors():
     assert abs(bench.col_rel_err(a, ref) - 0.1) < 1e-15
     assert bench.col_rel_err(ref, ref) == 0.0
     assert abs(bench.col_rel_err(np.array([2.0, 0.0]), np.array([1.0, 0.0])) - 1.0) < 1e-15
+
+
+def test_assembly_roofline_counts_what_is_integrated():
+    """Of two swapped element pairs one is integrated and the other copied, so
+    the achieved rate counts half of the evaluations off the diagonal."""
+    sys.path.insert(0, ROOT)
+    import bench
+    quad = {"regular": {"pairs": 6, "evaluations": 600}, "identical": {"pairs": 3, "evaluations": 900},
+            "edge": {"pairs": 4, "evaluations": 1000}, "vertex": {"pairs": 2, "evaluations": 400}}
+    r = bench.assembly_roofline(quad, 2.0, 1, 1e-6)
+    assert r["integrated"] == 900 + (600 + 1000 + 400) // 2
+    assert r["evaluations_per_s"] == r["integrated"] / 2.0
+    flops = r["integrated"] * bench.near_flops_per_evaluation(1)
+    assert abs(r["achieved"] - flops / 2.0 / 1e12) < 1e-20 and abs(r["frac"] - r["achieved"] / 1e-6) < 1e-12
