@@ -165,8 +165,6 @@ constexpr int kOzMinUnit = 30;
 // pairs: rows whose largest entry is below 2^-111 are split as if it were
 // that, which keeps the scale 2^(14 - e) a normal FP32 number
 constexpr int kMinPairExp = -110;
-// the row exponent of rows with Inf or NaN, which have no digits
-constexpr int kSpecialExp = 2047 - 1021;
 int oz_unit(int B, bool cplx, int max_row_blocks) {
   const long n = (long)std::max(1, max_row_blocks) * B * (cplx ? 2 : 1);
   int lg = 0;
@@ -444,10 +442,6 @@ __device__ __noinline__ uint32_t careful_columns(const OzArgs& a, const OzSeg& g
   const int ncol = min(16, min(per, a.ncols - pass * per) - first), c = first + (lane & 15);
   const int kb = g.row_ptr[row], ke = g.row_ptr[row + 1], ng = (a.B + 7) / 8;
   bool care = a.fmax[(pass * a.nseg + seg) * 32 + c] == 2047;
-  bool special = false;
-  if (kb < ke)
-    for (int i = lane; i < a.B; i += 32) special |= g.rexp[(long)row * a.B + i] == kSpecialExp;
-  care |= __any_sync(0xffffffffu, special);
   if (a.care > 0.0f && kb < ke) {
     float sum = 0.0f, most = 0.0f;
     for (int k = kb + (lane >> 4); k < ke; k += 2) {
@@ -545,8 +539,8 @@ __device__ void plain_columns(const OzArgs& a, const OzSeg& g, int row, int col0
 // with |A_ij| <= 2^(e - 1) over block row r. A thread owns one row of the
 // blocks and a share of their columns. spread, if given: the most that the
 // exponents of a row's entries (complex: of the larger parts) differ, with its
-// own value; 2047 where a row cannot be kept as digits: it holds Inf or NaN, or,
-// as complex couplings are kept as FP32 pairs, passes their range.
+// own value; at least 2046 in rows of complex couplings that FP32 pairs cannot
+// hold, and 2047 in rows with Inf or NaN.
 template <bool C>
 __global__ void k_oz_rows(const int* __restrict__ row_ptr, const double* __restrict__ blocks, long bstride, int B,
                           int* __restrict__ e, int* spread) {
@@ -578,8 +572,8 @@ __global__ void k_oz_rows(const int* __restrict__ row_ptr, const double* __restr
   __syncthreads();
   for (int t = threadIdx.x; t < B; t += blockDim.x) {
     e[(long)r * B + t] = top[t] - 1021;
-    const bool outside = top[t] == 2047 || (C && top[t] - 1023 > 126);
-    if (spread && kb < ke) atomicMax(spread, outside ? 2047 : top[t] - low[t]);
+    const int most = top[t] == 2047 ? 2047 : C && top[t] - 1023 > 126 ? 2046 : top[t] - low[t];
+    if (spread && kb < ke) atomicMax(spread, most);
   }
 }
 

@@ -1561,15 +1561,22 @@ extern "C" bg_status bg_operator_assemble(bg_operator* op) {
     }
     // digits (complex: row exponents) of the blocks for the FP64-accurate tensor-core product
     if (nb > 0 && op->near_oz) {
-      e = build_digits(op, op->dense, op->d_dense64.p, &op->d_dense_dig,
-                       op->cplx ? 0 : op->digit_bytes(nb, (int)B), op->near_tail(), nullptr);
+      int* spread = op->d_err.as<int>() + 1;
+      int most = 0;
+      e = cudaMemsetAsync(spread, 0, sizeof(int), op->ctx->stream);
+      if (e == cudaSuccess)
+        e = build_digits(op, op->dense, op->d_dense64.p, &op->d_dense_dig,
+                         op->cplx ? 0 : op->digit_bytes(nb, (int)B), op->near_tail(), spread);
       if (e == cudaSuccess) {
         const OzSeg g = oz_near_seg(op, op->d_dense64, op->d_dense_dig);
         e = launch_bsr_oz_floors(op->cplx, g.row_ptr, op->d_dense64.p, op->block_stride((int)B), op->dense.nrows, (int)B,
                                  g.rexp, const_cast<float*>(g.floors), op->ctx->stream);
       }
       if (e == cudaSuccess) e = cudaStreamSynchronize(op->ctx->stream);
+      if (e == cudaSuccess) e = cudaMemcpy(&most, spread, sizeof(int), cudaMemcpyDeviceToHost);
       if ((st = cuda_status(op->ctx, e, "near-field digits")) != BG_OK) return st;
+      // Inf or NaN have no digits: without them every product takes FP64 sums
+      if (most == 2047) op->d_dense_dig.release();
     }
   }
   auto t2 = std::chrono::steady_clock::now();

@@ -258,7 +258,7 @@ bool bsr_oz_supported(int B, bool cplx, bool pairs, int max_row_blocks);
 size_t bsr_oz_panel_bytes(int B, bool cplx);  // 0: block size not supported
 long bsr_oz_tile_stride(int B);               // bytes between the (real) blocks' digit bytes
 // row exponents [nrows B] of FP64 blocks (column-major, complex interleaved), digit bytes of real ones; spread, if
-// given, becomes the most that exponents differ within a row (2047: a row is outside the digits' range), or stays
+// given, becomes the most that exponents differ within a row (2047: Inf or NaN; 2046: not for FP32 pairs), or stays
 cudaError_t launch_bsr_oz_rows(bool cplx, const int* row_ptr, const void* blocks, long bstride, int nrows, int B,
                                int* rexp, int* spread, cudaStream_t s);
 cudaError_t launch_bsr_oz_tiles(const int* row_ptr, const double* blocks, long bstride, int nrows, int B,
