@@ -842,7 +842,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_bsr_oz(const __grid_constant_
   __shared__ uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_free[2], fin_bar;
   __shared__ uint64_t raw_full[kMaxRaws], raw_empty[kMaxRaws];
   __shared__ uint32_t tmem_slot;
-  __shared__ int abort_flag, any_careful;
+  __shared__ int abort_flag, any_careful, conv_left, conv_stages[kConvWarps];
   volatile int* abort_v = &abort_flag;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int S = a.stages;
@@ -866,7 +866,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_bsr_oz(const __grid_constant_
       mbar_init(&acc_free[b], kEpiWarps);
     }
     mbar_init(&fin_bar, 1);
-    abort_flag = any_careful = 0;
+    abort_flag = any_careful = conv_left = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -883,6 +883,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_bsr_oz(const __grid_constant_
     const int u0 = 32 * (warp - kConvWarp0) + lane, jg0 = u0 / a.B, i0 = u0 - jg0 * a.B;
     Ring sr{0, 0u}, rr{0, 0u};
     int item = -1, ex0 = 0;  // the exponent of row i0 (pairs and FP64 entries are split here)
+    int stages = 0;          // handed over
     for (open_item(a, cur); !cur.done; next_stage<PARTS>(a, cur)) {
       const int slot = sr.slot, raw = rr.slot;
       const int* rexp = a.seg[cur.seg].rexp + (long)cur.row * a.B;
@@ -974,8 +975,14 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_bsr_oz(const __grid_constant_
         mbar_arrive(&full[slot]);
         if (last) mbar_arrive(&raw_empty[raw]);
       }
+      ++stages;
       sr.next(S);
       if (last) rr.next(a.raws);
+    }
+    if (lane == 0) {
+      conv_stages[warp - kConvWarp0] = stages;
+      __threadfence_block();
+      atomicAdd(&conv_left, 1);
     }
   } else if (warp == kTmaWarp) {
     // ---- copies: one thread fills the raw ring and the panel slots, each as
@@ -986,6 +993,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_bsr_oz(const __grid_constant_
       open_item(a, cr);
       open_item(a, cur);
       Ring rr{0, 0u}, sr{0, 0u};
+      int panels = 0;  // stages whose panels are under way or there
       long long t0 = clock64();
       while (!(cr.done && cur.done)) {
         bool moved = false;
@@ -1017,6 +1025,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_bsr_oz(const __grid_constant_
                      g.panels + (size_t)cur.pass * a.pass_panels + (size_t)__ldg(g.col + cur.k + b) * a.panel +
                          (size_t)cur.chunk * a.kw * a.nc * 8u * 32u,
                      bytes, &full[slot]);
+          ++panels;
           sr.next(S);
           next_stage<PARTS>(a, cur);
           moved = true;
@@ -1029,13 +1038,24 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_bsr_oz(const __grid_constant_
           break;
         }
       }
-      // after an abort, the copies still in flight land before the CTA exits:
-      // a panel's copy is waited for by its own barrier only where the
-      // converters arrived too, so the panels get time instead
+      // after an abort, the copies still in flight land before the CTA exits.
+      // A panel's barrier counts the converters' arrivals too: once they have
+      // left (their waits are bounded), this thread arrives for those that had
+      // not reached the stage, and the phase ends with the copy.
       if (*abort_v) {
         for (int q = 0; q < a.raws; ++q) mbar_wait(&raw_full[q], q < rr.slot ? rr.phase : rr.phase ^ 1u);
         const long long t1 = clock64();
-        while (clock64() - t1 < 2000000LL) {  // a millisecond, against microseconds for a copy
+        volatile int* left = &conv_left;
+        while (*left < kConvWarps && clock64() - t1 < 4 * kWaitCycles) {
+        }
+        if (*left == kConvWarps) {
+          __threadfence_block();
+          volatile int* done = conv_stages;
+          for (int n = max(0, panels - S); n < panels; ++n) {
+            for (int w = 0; w < kConvWarps; ++w)
+              if (done[w] <= n) mbar_arrive(&full[n % S]);
+            mbar_wait(&full[n % S], (uint32_t)(n / S) & 1u);
+          }
         }
       }
     }
