@@ -1652,6 +1652,41 @@ static cudaError_t oz_far_product(const bg_operator* op, const std::vector<DevBu
   return launch_bsr_oz(op->cplx, op->cplx, a, op->far_row_max, op->oz_far_passes, op->ctx->stream);
 }
 
+// Whether the FP64 far field goes through the digits
+static bool far_by_digits(const bg_operator* op, bool solver) {
+  return op->far_oz && !op->any_far_wide() && op->store_far && !(solver && op->maxwell());
+}
+// Digit panels of x for the FP64-accurate tensor-core products, and behind
+// them the marks of every block row, once a product comes that reads them: a
+// first product in another precision or of one column has not to wait for
+// their allocation (first mixed products of one column: sphere M = 2, P = 1 290
+// -> 236 us, torus M = 1, P = 2 358 -> 250; the product itself takes 150 and 200).
+static bg_status ensure_digits(bg_operator* op, int nrhs, int prec, bool solver) {
+  const int nr = op->kbatched() ? nrhs / (int)op->kslots.size() : nrhs;
+  bool near = near_by_digits(op, op->d_dense_dig, nr, solver);
+  if (op->kbatched())
+    for (const auto& k : op->kslots) near |= near_by_digits(op, k.dense_dig, nr, solver);
+  near &= prec != BG_PREC_FP32;
+  const bool far = prec == BG_PREC_FP64 && far_by_digits(op, solver);
+  auto grow = [&](DevBuf* b, size_t one, int passes, int* have) -> bg_status {
+    if (b->p && *have >= passes) return BG_OK;
+    if (b->p) op->drop_graphs();  // the panels move
+    BG_CHECK(b->alloc(one * passes), "digit panels");
+    *have = passes;
+    return BG_OK;
+  };
+  bg_status st = BG_OK;
+  if (near && (st = grow(&op->w_oz_near, (size_t)op->dense.nrows * oz_scratch(op->dense.B, op->cplx),
+                         oz_passes(op, op->dense.nrows, nr), &op->oz_near_passes)) != BG_OK)
+    return st;
+  const int cols = op->maxwell() ? 4 * std::min(nr, (int)bg_operator::kMwRhsChunk) : nr;
+  if (far && (st = grow(&op->w_oz_far, oz_far_panels(op, nullptr) + (size_t)op->n_far_work * kOzMarks,
+                        oz_passes(op, op->n_far_work, cols), &op->oz_far_passes)) != BG_OK)
+    return st;
+  if (near || far) BG_CHECK(op->w_oz_fmax.alloc((size_t)2 * kOzFmax * sizeof(int)), "digit panels");
+  return BG_OK;
+}
+
 bg_status ensure_work(bg_operator* op, int nrhs) {
   if (nrhs <= op->cap) return BG_OK;
   op->drop_graphs();  // the buffers below move
@@ -1690,20 +1725,6 @@ bg_status ensure_work(bg_operator* op, int nrhs) {
       BG_CHECK(op->w_btiles[l]->alloc(tb * op->nclusters(l)), "work vectors");
       BG_CHECK(op->w_binv[l]->alloc(sizeof(float) * 32 * op->nclusters(l)), "work vectors");
     }
-  }
-  // digit panels of x for the FP64-accurate tensor-core products, and behind
-  // them the marks of every block row
-  {
-    op->oz_near_passes = oz_passes(op, op->dense.nrows, nrhs);
-    if (op->near_oz)
-      BG_CHECK(op->w_oz_near.alloc((size_t)op->dense.nrows * oz_scratch(op->dense.B, op->cplx) * op->oz_near_passes),
-               "work vectors");
-    const int cols = op->maxwell() ? 4 * std::min(nrhs, (int)bg_operator::kMwRhsChunk) : nrhs;
-    op->oz_far_passes = oz_passes(op, op->n_far_work, cols);
-    if (op->far_oz)
-      BG_CHECK(op->w_oz_far.alloc((oz_far_panels(op, nullptr) + (size_t)op->n_far_work * kOzMarks) * op->oz_far_passes),
-               "work vectors");
-    BG_CHECK(op->w_oz_fmax.alloc((size_t)2 * kOzFmax * sizeof(int)), "work vectors");
   }
   if (op->fmm_fused) {
     // arrival counters of the fused upward pass: parents at levels
@@ -2069,7 +2090,7 @@ static bg_status apply_middle(bg_operator* op, int nrhs, int prec, bool solver, 
       return BG_OK;
     };
     // FP64 far field on the tensor cores, all levels in one launch
-    const bool oz_far = !mixed && op->far_oz && !op->any_far_wide() && op->store_far && !(solver && op->maxwell());
+    const bool oz_far = !mixed && far_by_digits(op, solver);
     if (oz_far && op->maxwell()) {
       const std::complex<double> kap(op->kre, op->kim), mk2 = -1.0 / (kap * kap);
       for (int r0 = 0; r0 < nrhs; r0 += bg_operator::kMwRhsChunk) {
@@ -2272,12 +2293,13 @@ bg_status apply_operator(bg_operator* op, int nrhs, int prec, const void* xdof, 
       BG_CHECK(op->kb_ys.alloc(blk), "near-field column blocks");
     }
   }
+  bg_status st = ensure_digits(op, nrhs, prec, solver);
+  if (st != BG_OK) return st;
   cudaStream_t s = op->ctx->stream;
   const int S64 = op->stype(false);
   BG_CHECK(timed_launch(op->ctx, KC_TAPPLY, [&] { return launch_csr_apply(S64, op->d_T_ptr.as<int>(), op->d_T_idx.as<int>(), op->d_T_val.as<double>(), op->S, xdof,
                             op->w_xss.p, nrhs, s); }),
            "T x");
-  bg_status st = BG_OK;
   bg_context* ctx = op->ctx;
   if (ctx->profiling || !op->use_graphs) {
     st = apply_middle(op, nrhs, prec, solver);
@@ -2376,6 +2398,7 @@ extern "C" bg_status bg_operator_autotune(bg_operator* op, int nrhs, int precisi
   cudaSetDevice(ctx->device);
   cudaStream_t s = ctx->stream;
   bg_status st = ensure_work(op, nrhs);
+  if (st == BG_OK) st = ensure_digits(op, nrhs, precision, false);
   if (st != BG_OK) return st;
   // seeded superspace input in [-1, 1) (a 64-bit linear congruential generator)
   std::vector<double> x((size_t)op->S * nrhs * (op->cplx ? 2 : 1));

@@ -383,3 +383,38 @@ def test_operators_with_infinities(ctx, tmp_path, geo, M, kind, kappa, np_):
         d.compute()
         y = d.get_discrete_operator().matvec(x)
         assert np.linalg.norm(y - clean) < 1e-13 * np.linalg.norm(clean)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+def test_digit_panels_come_with_the_products_that_read_them(ctx, kind):
+    """The digit panels of x are allocated by the first product that reads them
+    (near field: mixed and FP64, far field: FP64), so that the first product of
+    another kind does not wait for them; whatever the order of the precisions
+    and column counts, also over graphs that the growing panels make stale,
+    results have the bits of an operator that starts with the largest."""
+    import ctypes
+    from bembel_gb300 import _lib
+
+    def allocated(d):
+        a, e = ctypes.c_size_t(), ctypes.c_size_t()
+        ctx.check(_lib.load().bg_operator_memory(d.h, ctypes.byref(a), ctypes.byref(e)))
+        return a.value
+
+    d, whole = (_operator(ctx, SPHERE, 2, 1, kind, 1.3) for _ in range(2))
+    assert d.n_lowrank > 0
+    rng = np.random.default_rng(21)
+    x = rng.normal(size=(d.N, 70)) + (1j * rng.normal(size=(d.N, 70)) if kind else 0)
+    ref = {n: whole.get_discrete_operator().matvec(x[:, :n]) for n in (70, 40, 5)}
+    mixed = whole.get_discrete_operator().matvec(x[:, :5], precision="mixed")
+    A = d.get_discrete_operator()
+    A.matvec(x[:, :5], precision="fp32")
+    m = [allocated(d)]
+    for prec in ("mixed", "fp64"):
+        for _ in range(3):
+            assert np.array_equal(A.matvec(x[:, :5], precision=prec), mixed if prec == "mixed" else ref[5])
+        m.append(allocated(d))
+    assert m[0] < m[1] < m[2]
+    for n in (40, 5, 70, 40):
+        for _ in range(2):
+            assert np.array_equal(A.matvec(x[:, :n]), ref[n]), n
+    assert np.array_equal(A.matvec(x[:, :5], precision="mixed"), mixed)
