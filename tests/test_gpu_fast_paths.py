@@ -418,3 +418,48 @@ def test_digit_panels_come_with_the_products_that_read_them(ctx, kind):
         for _ in range(2):
             assert np.array_equal(A.matvec(x[:, :n]), ref[n]), n
     assert np.array_equal(A.matvec(x[:, :5], precision="mixed"), mixed)
+
+
+@pytest.mark.parametrize("mcl", [0, 2])
+@pytest.mark.parametrize("geo,M,P,kind", [(SPHERE, 2, 1, 0), (TORUS, 2, 1, 1), (SPHERE, 2, 2, 1)])
+@pytest.mark.parametrize("prepared", [False, True])
+def test_mirrored_element_pairs_of_other_leaves(ctx, oracle, geo, M, P, kind, mcl, prepared):
+    """The copies of swapped pairs with one element and with 16 per leaf
+    cluster (pairs across leaves only, and mostly within one), assembled for
+    one wavenumber and prepared with a second one: every leaf block matches
+    the oracle to 1e-12, the parity bound."""
+    if prepared and not kind:
+        pytest.skip("no wavenumber to prepare")
+    d = _operator(ctx, geo, M, P, kind, 1.4, min_cluster_level=mcl)
+    if prepared:
+        d.prepare_wavenumbers([0.6, 2.2])
+        d.lin_op.set_wavenumber(2.2)
+        d.compute()
+    o = oracle.Problem(geo, M, P, kind, kappa=(2.2 if prepared else 1.4) if kind else 0.0, np_=6, mcl=mcl)
+    dense = [i for i, lv in enumerate(d.leaves()) if lv[0] == 2]
+    assert dense
+    for li in dense:
+        a, b = d.leaf_block(li), o.leaf_matrix(li)
+        assert np.linalg.norm(a - b) <= FP64_TOL * np.linalg.norm(b), li
+
+
+@pytest.mark.parametrize("P,np_", [(1, 7), (2, 9)])
+@pytest.mark.parametrize("nr", [1, 2, 3, 17])
+def test_batched_wavenumber_products_of_few_columns(ctx, P, np_, nr):
+    """Products of three batched wavenumbers, whose digit products read and
+    write a column block of wider rows, equal each wavenumber's own operator's
+    around the column counts at which the near field changes its kernel and a
+    pass is full (1e-13 for FP64, 1e-12 for mixed, as for other counts)."""
+    ks = [0.7, 2.0, 3.5 - 0.2j]
+    d = _operator(ctx, SPHERE, 2, P, 1, ks[0], np_)
+    d.prepare_wavenumbers(ks)
+    d.assemble_wavenumbers()
+    rng = np.random.default_rng(20)
+    x = rng.normal(size=(d.N, 3 * nr)) + 1j * rng.normal(size=(d.N, 3 * nr))
+    y = {prec: d.get_discrete_operator().matvec(x, precision=prec) for prec in ("fp64", "mixed")}
+    for q, k in enumerate(ks):
+        A = _operator(ctx, SPHERE, 2, P, 1, k, np_).get_discrete_operator()
+        cols = slice(q * nr, (q + 1) * nr)
+        for prec, tol in (("fp64", 1e-13), ("mixed", 1e-12)):
+            ref = A.matvec(x[:, cols], precision=prec)
+            assert np.linalg.norm(y[prec][:, cols] - ref) < tol * np.linalg.norm(ref), (prec, q)
