@@ -1145,9 +1145,9 @@ static bg_status assemble_near_mw(bg_operator* op) {
 // (e1, e2) to rounding (2e-15 in the oracle). With `mirror`, pairs e1 > e2
 // whose swapped pair is classified alike (case, degree and orientations) are
 // left out of the rules and copied instead (mirrored: transposed copy).
-// Maxwell's pairs are all integrated: its solves with an FP32 inner operator
-// turn a change of 1e-16 in the blocks into one of the stopping residual's
-// size in x.
+// Maxwell's pairs are all integrated (its blocks would have to swap components
+// too): its solves, which turn a change of 1e-16 in the blocks into one of the
+// stopping residual's size in x, keep the solutions that were.
 struct NearWork {
   std::map<int, std::vector<NearPair>> regular;
   std::map<std::pair<int, int>, std::vector<NearPair>> singular;
@@ -1550,8 +1550,9 @@ extern "C" bg_status bg_operator_assemble(bg_operator* op) {
                                 op->block_stride32((int)B), B * B, nb, op->ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(op->ctx->stream);
     if ((st = cuda_status(op->ctx, e, "FP32 near field")) != BG_OK) return st;
-    // (hi, lo) FP32 pairs of the real blocks: the FP64-accurate near field of
-    // BG_PREC_MIXED products runs on the FP32 pipes
+    // (hi, lo) FP32 pairs of the real blocks: BG_PREC_MIXED products take them
+    // where the digits do not apply and with a plan of mixed_near 1 or 2, which
+    // may be set at any time
     if (!op->cplx && nb > 0) {
       const long n = nb * op->block_stride((int)B);
       e = op->d_dense_df.alloc((size_t)n * sizeof(float2));

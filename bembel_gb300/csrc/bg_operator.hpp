@@ -370,9 +370,10 @@ bg_status check_device_flag(bg_operator* op);
 // field plus the FP32 fused far field (forward/backward transforms in FP32);
 // BG_PREC_FP32 as MIXED with the near field in FP32 as well.
 // solver: a product inside bg_solve. Maxwell's keep the double-float far field
-// and the FP64-pipe near field there: its flexible GMRES with an FP32 inner
-// solve turns differences of 1e-16 in the products into differences of the
-// stopping residual's size in x (1.5e-9 of the field at a tolerance of 1e-8,
-// against 1e-10 for the scalar operators), and its solves are to stay
-// reproducible.
+// and the FP64-pipe near field there, with every inner solve. Any Krylov solve
+// turns differences of 1e-16 in its products into differences of the stopping
+// residual's size in x; Maxwell's with an FP32 inner solve are the largest seen
+// (1.5e-9 of the field at a tolerance of 1e-8, against 1e-10 for the scalar
+// operators). The tolerance allows either; the older sums keep the solutions
+// that were, at the cost of slower products than bg_matvec's.
 bg_status apply_operator(bg_operator* op, int nrhs, int prec, const void* xdof, void* ydof, bool solver = false);

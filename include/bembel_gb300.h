@@ -282,7 +282,8 @@ bg_status bg_watchdog_selftest(bg_context* ctx, long long limit_cycles);
 /* ---- launch plans and the autotuner (no reference counterpart) ----
  * A launch plan fixes the kernel variants and schedules of the H2 product for
  * one (number of right-hand sides, precision). Products with no plan set use
- * the built-in choices ({0, -1, 0}). The FP64 product has no choices. */
+ * the built-in choices (0 everywhere, split_k_batches -1). Of these the FP64
+ * product reads `transforms` only. */
 typedef struct bg_launch_plan {
   /* FP32 near field (BG_PREC_FP32): 0 built-in choice; 1 the pipelined block
    * kernel; 2 register tiles (complex: 2 block rows per thread); 3 complex
@@ -309,8 +310,10 @@ typedef struct bg_launch_plan {
   int far_ctas;
   /* FP64-accurate near field of BG_PREC_MIXED products: 0 built-in (the
    * tensor-core product on 8 integer digits of 7 bits per operand, exact
-   * integer accumulation, which the FP64 product uses too, or for one or two
-   * columns the FP64 pipe); real operators also 1 double-float on the FP32
+   * integer accumulation, which the FP64 product uses too; the FP64 pipe for
+   * one column, for two real columns where leaf blocks have at most 16 rows,
+   * for leaf blocks of more than 128 rows and for near fields with Inf or
+   * NaN); real operators also 1 double-float on the FP32
    * pipes, 2 the double-float product with a quarter of 32 columns on the
    * FP64 pipe (32 columns only, else 1). All agree with the FP64 product to
    * about 1e-14 relative or better. */
