@@ -1605,10 +1605,13 @@ static size_t oz_far_panels(const bg_operator* op, size_t* off) {
 // Whether a near-field product with nc columns goes through the digits. A
 // digit product costs about the same up to 32 columns (complex: 16) and three
 // small launches more; the FP64 pipe is quicker for a single vector, and for
-// two with small blocks (sphere M = 4, B = 36, one column: 43 against 68 us,
-// two: 69 against 68; M = 5, P = 1, B = 16: 31 and 48 against 124 us; torus
-// M = 3, complex, one column: 293 against 289 us, Maxwell sphere M = 3: 150
-// against 177 us, two: 515 and 262 against 289 and 178 us).
+// two with small blocks, where there are many block rows (sphere M = 4, B = 36,
+// one column: 42 against 72 us, two: 69 against 71; M = 5, P = 1, B = 16: 30 and
+// 48 against 110 us; torus M = 3, complex, one column: 293 against 294 us,
+// Maxwell sphere M = 3: 151 against 182 us, two: 515 and 262 against 294 and 182
+// us). The rule does not look at the number of rows: with few of them the pipe
+// is kept where digits would be the quicker (sphere M = 2, B = 16, two columns
+// 32 against 26 us; complex, one column 51 against 38 us).
 static bool near_by_digits(const bg_operator* op, const DevBuf& dig, int nc, bool solver) {
   if (!op->near_oz || !dig.p || (solver && op->maxwell())) return false;
   return nc > 2 || (nc == 2 && (op->cplx || op->dense.B > 16));
