@@ -312,8 +312,8 @@ typedef struct bg_launch_plan {
    * tensor-core product on 8 integer digits of 7 bits per operand, exact
    * integer accumulation, which the FP64 product uses too; the FP64 pipe for
    * one column, for two real columns where leaf blocks have at most 16 rows,
-   * for leaf blocks of more than 128 rows and for near fields with Inf or
-   * NaN); real operators also 1 double-float on the FP32
+   * for near fields with Inf or NaN and for complex leaf blocks of more than
+   * 128 rows, where real ones take 1); real operators also 1 double-float on the FP32
    * pipes, 2 the double-float product with a quarter of 32 columns on the
    * FP64 pipe (32 columns only, else 1). All agree with the FP64 product to
    * about 1e-14 relative or better. */
