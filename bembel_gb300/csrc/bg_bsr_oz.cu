@@ -29,10 +29,15 @@
 // instead. The digits lose to it where S is small against 2^(e_i + f_c): an x of
 // very different sizes, a kernel that decays within the row.
 // Near field: the epilogue bounds S from below by the norms of x over 8 rows
-// and the floors of A over 8 columns, and marks the columns of a block row
+// and the floors of A over 8 columns and 36 rows, and marks the columns of a block row
 // where four times the digits' error could pass the plain sum's bound; the CTA
 // sums those in FP64 at its end (plain_columns). Columns of normal or smooth
-// values have S some 50 times above the line (B = 4 .. 64). All columns marked
+// values have S some 50 times above the line (B = 4 .. 64). Maxwell's blocks
+// (B = 72) hold small entries among the others, and with one floor for all their
+// rows half of the block rows had marks for normal x (sphere M = 3, mixed, 3
+// columns: floors 0.9 to 1.2 times the line, S 200 times; 305 -> 350 us). Two groups
+// of rows give 2.6 times and the old time back; at M = 4 (8 columns) most rows are
+// marked still, 1120 -> 2083 us. All columns marked
 // cost what the FP64 pipe did: sphere M = 5, P = 2, 32 columns 1.76 ms (1.49 on
 // the pipe, 0.23 unmarked), torus M = 3, 16 complex ones 2.03 (2.59, 0.30).
 // Far field: no row is marked. What an entry loses there is relative to the
@@ -443,25 +448,30 @@ __device__ __noinline__ uint32_t careful_columns(const OzArgs& a, const OzSeg& g
   const int kb = g.row_ptr[row], ke = g.row_ptr[row + 1], ng = (a.B + 7) / 8;
   bool care = a.fmax[(pass * a.nseg + seg) * 32 + c] == 2047;
   if (a.care > 0.0f && kb < ke) {
-    float sum = 0.0f, most = 0.0f;
-    for (int k = kb + (lane >> 4); k < ke; k += 2) {
-      const float* nx = reinterpret_cast<const float*>(g.panels + (size_t)pass * a.pass_panels +
-                                                       (size_t)g.col[k] * a.panel + oz_norms_at(a.nc, a.nks)) + c;
-      const float* fl = g.floors + (long)k * ng;
+    const int nh = oz_row_groups(a.B);
+    float least = FLT_MAX, most = 0.0f;
+    for (int r = 0; r < nh; ++r) {
+      float sum = 0.0f;
+      for (int k = kb + (lane >> 4); k < ke; k += 2) {
+        const float* nx = reinterpret_cast<const float*>(g.panels + (size_t)pass * a.pass_panels +
+                                                         (size_t)g.col[k] * a.panel + oz_norms_at(a.nc, a.nks)) + c;
+        const float* fl = g.floors + ((long)k * nh + r) * ng;
 #pragma unroll 4
-      for (int q = 0; q < ng; ++q) {
-        float v = nx[q * a.nc];
-        if (C) v = 0.7071f * (v + nx[q * a.nc + 16]);  // at most the sum of the moduli
-        sum = fmaf(fl[q], v, sum);
-        most = fmaxf(most, v);
+        for (int q = 0; q < ng; ++q) {
+          float v = nx[q * a.nc];
+          if (C) v = 0.7071f * (v + nx[q * a.nc + 16]);  // at most the sum of the moduli
+          sum = fmaf(fl[q], v, sum);
+          most = fmaxf(most, v);
+        }
       }
+      sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+      least = sum < least ? sum : (sum == sum ? least : sum);
     }
-    sum += __shfl_xor_sync(0xffffffffu, sum, 16);
     most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 16));
     const float n = (float)(ke - kb) * (float)(a.B * (C ? 2 : 1));
     const float roundings = (float)((ke - kb + a.chunk_blocks - 1) / a.chunk_blocks);  // of the fixed-point sum
     const float line = a.care * (0.15f * rsqrtf(n) + roundings * exp2f((float)(39 - a.unit)) / n);
-    care |= !(sum >= line) && most > 0.0f;
+    care |= !(least >= line) && most > 0.0f;
   }
   return __ballot_sync(0xffffffffu, care) & ((1u << max(ncol, 0)) - 1u);
 }
@@ -577,18 +587,19 @@ __global__ void k_oz_rows(const int* __restrict__ row_ptr, const double* __restr
   }
 }
 
-// floors[k][q]: lower bounds of |A_ij| 2^-e_i (complex: of the larger part) over
-// columns 8 q .. 8 q + 7 and all rows of block k. A warp per group of columns.
+// floors[k][r][q]: lower bounds of |A_ij| 2^-e_i (complex: of the larger part)
+// over columns 8 q .. 8 q + 7 and rows 36 r .. 36 r + 35 of block k. A warp per
+// group of columns and rows.
 template <bool C>
 __global__ void k_oz_floors(const int* __restrict__ row_ptr, const double* __restrict__ blocks, long bstride, int B,
                             const int* __restrict__ e, float* __restrict__ floors) {
-  const int r = blockIdx.x, ng = (B + 7) / 8, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int kb = row_ptr[r], n = (row_ptr[r + 1] - kb) * ng;
+  const int r = blockIdx.x, ng = (B + 7) / 8, per = ng * oz_row_groups(B), lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int kb = row_ptr[r], n = (row_ptr[r + 1] - kb) * per;
   for (int u = threadIdx.x >> 5; u < n; u += nw) {
-    const long k = kb + u / ng;
-    const int j0 = 8 * (u % ng), nv = min(8, B - j0);
+    const long k = kb + u / per;
+    const int j0 = 8 * (u % ng), nv = min(8, B - j0), i0 = kOzGroupRows * (u % per / ng);
     float m = FLT_MAX;
-    for (int i = lane; i < B; i += 32) {
+    for (int i = i0 + lane; i < min(B, i0 + kOzGroupRows); i += 32) {
       const int ei = e[(long)r * B + i];
       for (int c = 0; c < nv; ++c) {
         const long o = k * bstride + (long)(j0 + c) * B + i;
@@ -601,7 +612,7 @@ __global__ void k_oz_floors(const int* __restrict__ row_ptr, const double* __res
       }
     }
     const int bits = __reduce_min_sync(0xffffffffu, __float_as_int(m));  // not negative: ordered as integers
-    if (lane == 0) floors[k * ng + u % ng] = __int_as_float(bits);
+    if (lane == 0) floors[kb * (long)per + u] = __int_as_float(bits);
   }
 }
 

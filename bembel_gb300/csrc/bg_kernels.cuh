@@ -228,7 +228,8 @@ struct OzSeg {
   const unsigned char* tiles;  // block k at + k tstride bytes (pairs of Im: im_off bytes further)
   long tstride, im_off;
   const int* rexp;             // row exponents [rows][B]
-  const float* floors;         // care: [blocks][ceil(B / 8)], lower bounds of |A_ij| 2^-e_i over 8 columns, all rows
+  const float* floors;         // care: [blocks][oz_row_groups(B)][ceil(B / 8)], lower bounds of |A_ij| 2^-e_i over 8
+                               // columns and the rows of a group
   const double* exact;         // digit bytes: the FP64 blocks they came from, exact_stride apart; nullptr: not kept
   long exact_stride;
   const double* x;             // [ncl B][ldx] (complex interleaved)
@@ -256,6 +257,9 @@ struct OzArgs {
 // max_row_blocks: the longest block row; pairs: complex blocks as FP32 pairs, not FP64
 bool bsr_oz_supported(int B, bool cplx, bool pairs, int max_row_blocks);
 size_t bsr_oz_panel_bytes(int B, bool cplx);  // 0: block size not supported
+// groups of rows of a block with floors of their own
+constexpr int kOzGroupRows = 36;
+__host__ __device__ constexpr int oz_row_groups(int B) { return (B + kOzGroupRows - 1) / kOzGroupRows; }
 long bsr_oz_tile_stride(int B);               // bytes between the (real) blocks' digit bytes
 // row exponents [nrows B] of FP64 blocks (column-major, complex interleaved), digit bytes of real ones; spread, if
 // given, becomes the most that exponents differ within a row (2047: Inf or NaN; 2046: not for FP32 pairs), or stays

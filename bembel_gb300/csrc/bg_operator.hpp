@@ -345,7 +345,7 @@ struct bg_operator {
   }
   // bytes of the near field's row exponents and floors, which follow them
   size_t near_tail() const {
-    return (size_t)dense.nrows * dense.B * sizeof(int) + dense.col.size() * (size_t)((dense.B + 7) / 8) * sizeof(float);
+    return (size_t)dense.nrows * dense.B * sizeof(int) + dense.col.size() * (size_t)(bg::oz_row_groups(dense.B) * ((dense.B + 7) / 8)) * sizeof(float);
   }
   int stype(bool fp32) const { return (fp32 ? 2 : 0) + (cplx ? 1 : 0); }
   // Maxwell: the far field is stored as the scalar kernel matrix of each

@@ -463,3 +463,21 @@ def test_batched_wavenumber_products_of_few_columns(ctx, P, np_, nr):
         for prec, tol in (("fp64", 1e-13), ("mixed", 1e-12)):
             ref = A.matvec(x[:, cols], precision=prec)
             assert np.linalg.norm(y[prec][:, cols] - ref) < tol * np.linalg.norm(ref), (prec, q)
+
+
+@pytest.mark.parametrize("kind,kappa", [(0, 0), (1, 2.0), (1, 2.0 - 30.0j)])
+def test_digit_near_field_of_large_blocks_keeps_every_entry(ctx, kind, kappa):
+    """Leaf blocks of 64 rows, whose floors are kept by two groups of rows:
+    entry by entry the bound of plain FP64 sums, as for smaller blocks."""
+    d = _operator(ctx, SPHERE, 1, 3, kind, kappa)
+    assert d.n_lowrank == 0
+    T, A = _fp64_dense(d)
+    x = _spread_columns(d, T, np.random.default_rng(21), bool(kind))
+    wide = np.clongdouble if kind else np.longdouble
+    Tw = T.astype(np.longdouble)
+    ref = Tw.T @ (A.astype(wide) @ (Tw @ x.astype(wide)))
+    bound = np.abs(T).T @ (np.abs(A) @ (np.abs(T) @ np.abs(x)))
+    n = d.S * (2 if kind else 1)
+    err = np.abs(d.get_discrete_operator().matvec(x) - ref).astype(float)
+    assert (err <= (2 if kind else 1) * (n + 20) * 2.0 ** -53 * bound).all(), \
+        (err / np.maximum(bound, 1e-300)).max(axis=0)
