@@ -36,8 +36,9 @@
 // (B = 72) hold small entries among the others, and with one floor for all their
 // rows half of the block rows had marks for normal x (sphere M = 3, mixed, 3
 // columns: floors 0.9 to 1.2 times the line, S 200 times; 305 -> 350 us). Two groups
-// of rows give 2.6 times and the old time back; at M = 4 (8 columns) most rows are
-// marked still, 1120 -> 2083 us. All columns marked
+// of rows give 2.6 times and the old time back. At M = 4 (8 columns) the product
+// still takes 2083 us, 1120 without the fallback; groups of 4 rows do not change
+// that (2089), so its cause is another one, not found yet. All columns marked
 // cost what the FP64 pipe did: sphere M = 5, P = 2, 32 columns 1.76 ms (1.49 on
 // the pipe, 0.23 unmarked), torus M = 3, 16 complex ones 2.03 (2.59, 0.30).
 // Far field: no row is marked. What an entry loses there is relative to the
